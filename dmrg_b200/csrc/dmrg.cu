@@ -300,7 +300,7 @@ static int dmrg_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, DmrgW
                 g.M = (int)(d * ca), g.N = (int)(d * cb), g.K = (int)cc, g.batch = 1;
                 g.A = ws.M[i], g.lda = d * ca, g.B = ws.P2, g.ldb = cc, g.C = ws.Cbuf, g.ldc = d * ca;
                 g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
-                HEFF_TRY(gemm_f64<false>(false, false, false, g, s));
+                HEFF_TRY(gemm_f64<false>(false, false, g, s));
                 merge_layout_kernel<<<g1(d * d * ca * cb), 256, 0, s>>>(ws.Cbuf, ws.theta, d, ca, cb);
                 HEFF_LAUNCH_CHECK();
                 // eigensolve on the rebound operator
@@ -387,7 +387,7 @@ static int dmrg_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, DmrgW
         g.M = (int)(d * ca), g.N = (int)(d * cb), g.K = (int)cc, g.batch = 1;
         g.A = ws.M[0], g.lda = d * ca, g.B = ws.P2, g.ldb = cc, g.C = ws.Cbuf, g.ldc = d * ca;
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
-        HEFF_TRY(gemm_f64<false>(false, false, false, g, s));
+        HEFF_TRY(gemm_f64<false>(false, false, g, s));
         merge_layout_kernel<<<g1(d * d * ca * cb), 256, 0, s>>>(ws.Cbuf, ws.theta, d, ca, cb);
         HEFF_LAUNCH_CHECK();
         // Lenv[0] still holds the trivial left edge (1)
@@ -486,7 +486,7 @@ static int gemm_nn(const double *A, int64_t lda, const double *B, int64_t ldb, d
     g.M = (int)M, g.N = (int)N, g.K = (int)K, g.batch = 1;
     g.A = A, g.lda = lda, g.B = B, g.ldb = ldb, g.C = C, g.ldc = ldc;
     g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
-    return gemm_f64<false>(false, false, false, g, s);
+    return gemm_f64<false>(false, false, g, s);
 }
 
 // A (m x n, lda) = U S VT with U m x k (ld m), VT k x n (ld k); the one-sided Jacobi always runs on the taller

@@ -307,9 +307,9 @@ struct Davidson {
         g.M = (int)n, g.N = m, g.K = k, g.batch = 1;
         g.A = V, g.lda = n, g.B = dc, g.ldb = k, g.C = V2, g.ldc = n;
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
-        HEFF_TRY(gemm_f64<CPLX>(false, false, false, g, s));
+        HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
         g.A = AV, g.C = AV2;
-        HEFF_TRY(gemm_f64<CPLX>(false, false, false, g, s));
+        HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
         std::swap(V, V2);
         std::swap(AV, AV2);
         if(track_g2) {  // G2 <- S^H G2 S

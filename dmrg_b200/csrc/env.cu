@@ -133,7 +133,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         g.B = Mc, g.ldb = cL, g.sB = 0;
         g.C = X, g.ldc = cL, g.sC = cL * d * cR;
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
-        HEFF_TRY(gemm_f64<CPLX>(false, false, false, g, s));
+        HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
         if(cR > 65535) return HEFF_BAD_SHAPE;
         dim3 grid((unsigned)cdiv(cL, 128), (unsigned)cR);
         env_mix_kernel<T, true><<<grid, 128, wsm, s>>>(X, Y, W, (int)d, (int)cL, (int)cR, (int)DL, (int)DR);
@@ -143,7 +143,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         h.A = M, h.lda = d * cL, h.B = Y, h.ldb = d * cL, h.C = out, h.ldc = cR;
         h.alpha = make_double2(1, 0), h.beta = make_double2(0, 0);
         h.split_ws = split_ws, h.split_ws_bytes = split_bytes;
-        HEFF_TRY(gemm_f64<CPLX>(true, false, false, h, s));
+        HEFF_TRY(gemm_f64<CPLX>(true, false, h, s));
     } else {
         env_prep_R<<<grid1(nM), 256, 0, s>>>(M, Mc, M2, d, cL, cR, nM);
         HEFF_LAUNCH_CHECK();
@@ -153,7 +153,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         g.B = Mc, g.ldb = d * cL, g.sB = 0;  // conj(M) stored N x K: (s',a') contiguous, b' outer
         g.C = X, g.ldc = cR, g.sC = cR * d * cL;
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
-        HEFF_TRY(gemm_f64<CPLX>(false, true, false, g, s));
+        HEFF_TRY(gemm_f64<CPLX>(false, true, g, s));
         if(cL > 65535) return HEFF_BAD_SHAPE;
         dim3 grid((unsigned)cdiv(cR, 128), (unsigned)cL);
         env_mix_kernel<T, false><<<grid, 128, wsm, s>>>(X, Y, W, (int)d, (int)cR, (int)cL, (int)DL, (int)DR);
@@ -163,7 +163,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         h.A = M2, h.lda = d * cR, h.B = Y, h.ldb = d * cR, h.C = out, h.ldc = cL;
         h.alpha = make_double2(1, 0), h.beta = make_double2(0, 0);
         h.split_ws = split_ws, h.split_ws_bytes = split_bytes;
-        HEFF_TRY(gemm_f64<CPLX>(true, false, false, h, s));
+        HEFF_TRY(gemm_f64<CPLX>(true, false, h, s));
     }
     return HEFF_OK;
 }

@@ -103,7 +103,7 @@ int expansion_term(int side, typename Scalar<CPLX>::T *P, const typename Scalar<
     g.ldc   = S * cL;
     g.alpha = make_double2(alpha, 0.0);
     g.beta  = make_double2(0.0, 0.0);
-    HEFF_TRY(gemm_f64<CPLX>(false, false, false, g, s));
+    HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
     expansion_mix_R<T><<<ex_grid(nP), 256, smem, s>>>(X, W, P, (int)S, cL, cR, (int)DL, (int)DR);
     HEFF_LAUNCH_CHECK();
     return HEFF_OK;

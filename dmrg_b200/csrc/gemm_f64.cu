@@ -10,8 +10,8 @@
 
 namespace heff {
 
-// Tail-split mode of the DMMA GEMMs: 0 off, 1 automatic (the cost model below), 2..16 that many pieces whenever
-// the tiles leave a partial wave.  Initial value from the environment variable HEFF_GEMM_SPLIT (default 1).
+// Tail-split mode of the DMMA GEMMs: 0 no K split at all, 1 automatic (the cost model below), 2..16 that many pieces
+// whenever the large tiles leave a partial wave.  Initial value from the environment variable HEFF_GEMM_SPLIT (default 1).
 static std::atomic<int> g_split_mode{-1};
 
 static int split_mode() {
@@ -26,40 +26,9 @@ static int split_mode() {
     return m;
 }
 
-SplitPlan gemm_split_plan(int64_t tiles, int KT, int64_t slots, int64_t max_units, double tile_s, double unit_bytes) {
-    SplitPlan best;
-    best.nfull = (int)tiles;
-    const int mode = split_mode();
-    if(mode == 0 || slots <= 0 || tiles <= 0 || tiles % slots == 0 || tile_s <= 0) return best;
-    const int64_t waves = tiles / slots, rem = tiles % slots;
-    if(mode >= 2) {  // forced piece count (when the pieces keep >= 1 k-tile and fit the scratch)
-        if(KT >= mode && rem * mode <= max_units) {
-            best.split = mode;
-            best.nfull = (int)(tiles - rem);
-        }
-        return best;
-    }
-    // cost of a split in units of one whole tile's time: the reduction launch plus the partial tiles written
-    // and read back at HBM speed (device-wide)
-    constexpr double kLaunchS = 5e-6, kHbmBps = 6.0e12;
-    double           best_cost = (double)waves + 1.0;
-    for(int s = 2; s <= SPLIT_MAX; s++) {
-        if(KT / s < 4) break;
-        const int64_t units = rem * s;
-        if(units > max_units) break;
-        const double cost = (double)waves + (double)cdiv(units, slots) / s + (kLaunchS + 2.0 * unit_bytes * units / kHbmBps) / tile_s;
-        if(cost < best_cost - 1e-9) {
-            best_cost  = cost;
-            best.split = s;
-            best.nfull = (int)(tiles - rem);
-        }
-    }
-    return best;
-}
-
 size_t gemm_split_ws_bytes() {
     // at most 4 partial tiles per co-resident CTA (the real kernel runs one 128x128 CTA per SM)
-    return (size_t)4 * device_sm_count() * GemmTile<false>::BM * GemmTile<false>::BN * sizeof(double);
+    return (size_t)4 * device_sm_count() * GemmTile<false, 0>::BM * GemmTile<false, 0>::BN * sizeof(double);
 }
 
 // Every DMMA GEMM kernel (and split reduction) this process has launched; a captured graph's kernel nodes are
@@ -75,93 +44,163 @@ bool gemm_fn_known(const void *f) {
     return std::find(g_gemm_fns.begin(), g_gemm_fns.end(), f) != g_gemm_fns.end();
 }
 
-template<bool CPLX, bool TA, bool TB, bool CJA, int VEC>
-static int launch_gemm(const GemmArgs &a_in, cudaStream_t stream) {
-    using G                  = GemmTile<CPLX>;
-    using SM                 = GemmSmem<CPLX, TA, TB>;
-    using T                  = typename Scalar<CPLX>::T;
-    auto       kern = gemm_f64_kernel<CPLX, TA, TB, CJA, VEC>;
+// How a GEMM runs: tile shape; K pieces of every tile on a cluster (cluster > 1); or K pieces of the tiles of the last
+// partial wave, from tile nfull on, summed by a second kernel (split > 1).  Tiles count over all batch members.
+struct GemmPlan {
+    int     cfg = 0, cluster = 1, split = 1;
+    int64_t nfull = 0;
+    double  cost  = 0;
+};
+
+struct TileShape {
+    int    bm, bn, bk, occ;  // co-resident CTAs per SM
+    double full, alone;      // sustained fraction of the DMMA rate: SM full of such CTAs, one CTA alone on its SM
+};
+template<bool CPLX>
+static const TileShape &tile_shape(int cfg) {
+    static const TileShape r[3] = {{128, 128, 32, 1, 0.95, 0.95}, {64, 64, 32, 1, 0.92, 0.92}, {32, 32, 32, 3, 0.86, 0.62}};
+    static const TileShape c[2] = {{64, 64, 32, 1, 0.87, 0.87}, {32, 32, 32, 2, 0.82, 0.65}};
+    return CPLX ? c[cfg] : r[cfg];
+}
+
+// Plan of one problem: the smallest estimate over tile shapes and K splits.  An SM does 64 DMMA FMAs per clock
+// whatever the tile, so a variant's time is the busiest SM's share of the padded products at the rate its tile sustains
+// (tile_shape), plus what its launches cost.  The constants come from a sweep of every variant over the matvec and
+// environment GEMMs of chi = 8 .. 1024 (real / complex): a GEMM of one k-tile takes 4.2 us back to back, a cluster of 2
+// or 4 adds 3.6 us (8 adds 7 and never won), the reduction kernel of a tail split 5 us.  Examples, us for (whole tiles
+// of 128/64/32 | best): f64 96x128x32 10.3/6.2/4.2 | 4.2; f64 1024x256x768 109/31/18.5 | 18.5; c128 192x128x384
+// -/49/18.5 | 10.3 (cluster of 4); f64 3072x4096x1024 840/-/- | 743 (tail split).
+template<bool CPLX>
+static GemmPlan gemm_pick(const GemmArgs &a) {
+    constexpr double kClk = 1.9e9, kLaunch = 3.2e-6, kCluster = 3.6e-6, kReduce = 5e-6, kHbm = 6.0e12;
+    const int     mode = split_mode(), sms = device_sm_count();
+    const double  fma  = CPLX ? 3.0 : 1.0;
+    GemmPlan      best;
+    bool          have = false;
+    for(int cfg = 0; cfg < gemm_cfgs(CPLX); cfg++) {
+        if(mode >= 2 && cfg > 0) break;  // forced tail split: the large tiles
+        const TileShape &t     = tile_shape<CPLX>(cfg);
+        const int64_t    tiles = cdiv(a.M, t.bm) * cdiv(a.N, t.bn) * a.batch, KT = cdiv(a.K, t.bk);
+        const double     kt_s  = (double)t.bm * t.bn * t.bk * fma / 64.0 / kClk;  // one k-tile at the full DMMA rate
+        auto             rate  = [&](int64_t units) {
+            const int64_t per = std::min<int64_t>(cdiv(units, sms), t.occ);
+            return t.occ > 1 ? t.alone + (t.full - t.alone) * (double)(per - 1) / (t.occ - 1) : t.full;
+        };
+        for(int ks = 1; ks <= CLUSTER_MAX; ks *= 2) {
+            const int64_t units = tiles * ks;
+            // clusters are placed within a GPC: with one CTA per SM, a quarter of the SMs can stay out of reach of them
+            if(ks > 1 && (mode != 1 || ks > KT || units > (t.occ > 1 ? sms : 3 * sms / 4))) break;
+            GemmPlan q;
+            q.cfg = cfg, q.cluster = ks, q.nfull = tiles;
+            q.cost = kLaunch + (double)(cdiv(units, sms) * cdiv(KT, ks)) * kt_s / rate(units) + (ks > 1 ? kCluster : 0.0);
+            if(!have || q.cost < best.cost) best = q, have = true;
+        }
+        if(t.occ == 1 && a.split_ws && mode >= 1 && tiles % sms != 0) {
+            const double  unit_bytes = (double)t.bm * t.bn * (CPLX ? 16.0 : 8.0);
+            const int64_t rem = tiles % sms, max_units = (int64_t)((double)a.split_ws_bytes / unit_bytes);
+            for(int sp = mode >= 2 ? mode : 2; sp <= (mode >= 2 ? mode : SPLIT_MAX); sp++) {
+                if(rem * sp > max_units || KT < (mode >= 2 ? sp : 4 * sp)) break;
+                GemmPlan q;
+                q.cfg = cfg, q.split = sp, q.nfull = tiles - rem;
+                q.cost = kLaunch + (double)(tiles / sms * KT + cdiv(rem * sp, sms) * cdiv(KT, sp)) * kt_s / rate(tiles - rem + rem * sp) + kReduce +
+                         2.0 * unit_bytes * (double)(rem * sp) / kHbm;
+                if(q.cost < best.cost || mode >= 2) best = q;
+            }
+        }
+    }
+    return best;
+}
+
+template<bool CPLX, int CFG, bool TA, bool TB, int VEC>
+static int launch_gemm(const GemmArgs &a_in, const GemmPlan &pl, cudaStream_t stream) {
+    using G                  = GemmTile<CPLX, CFG>;
+    using SM                 = GemmSmem<CPLX, CFG, TA, TB>;
+    auto       kern = gemm_f64_kernel<CPLX, CFG, TA, TB, VEC>;
     static int occ[64] = {0};  // per instantiation and device: co-resident CTAs per SM (0 = not set up yet)
     int        dev     = 0;
     HEFF_CUDA(cudaGetDevice(&dev));
     if(dev < 0 || dev >= 64 || !occ[dev]) {
         HEFF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::BYTES));
         int n = 0;
-        HEFF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, SM::BYTES));
+        HEFF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, G::THREADS, SM::BYTES));
         if(dev >= 0 && dev < 64) occ[dev] = n > 0 ? n : 1;
     }
     const int     per_sm = (dev >= 0 && dev < 64) ? occ[dev] : 1;
-    const int64_t tiles  = cdiv(a_in.M, G::BM) * cdiv(a_in.N, G::BN);
-    if(tiles > 0x7fffffffLL) return HEFF_BAD_SHAPE;
-    GemmArgs  a = a_in;
-    SplitPlan sp;
-    sp.nfull = (int)tiles;
-    if(a.split_ws && a.batch == 1) {
-        const int64_t tile_bytes = (int64_t)G::BM * G::BN * sizeof(T);
-        // one whole tile's time on one SM: its DMMA work (3 real products per complex one) at ~30 TFLOP/s per device
-        const double  sms    = (double)device_sm_count();
-        const double  tile_s = (CPLX ? 3.0 : 1.0) * 2.0 * G::BM * G::BN * (double)a.K / (30e12 / sms) * per_sm;
-        sp = gemm_split_plan(tiles, (int)cdiv(a.K, G::BK), (int64_t)device_sm_count() * per_sm, (int64_t)(a.split_ws_bytes / tile_bytes), tile_s,
-                             (double)tile_bytes);
-    }
-    a.split = sp.split;
-    a.nfull = sp.nfull;
-    a.part  = sp.split > 1 ? a.split_ws : nullptr;
-    const int64_t ctas = sp.nfull + (tiles - sp.nfull) * sp.split;
-    if(ctas > 0x7fffffffLL) return HEFF_BAD_SHAPE;
-    dim3 grid((unsigned)ctas, 1u, (unsigned)a.batch);
+    const int64_t tiles  = cdiv(a_in.M, G::BM) * cdiv(a_in.N, G::BN) * a_in.batch;
+    GemmArgs      a      = a_in;
+    const int64_t units  = pl.cluster > 1 ? tiles * pl.cluster : pl.nfull + (tiles - pl.nfull) * pl.split;
+    if(tiles > 0x3fffffffLL || units > 0x3fffffffLL) return HEFF_BAD_SHAPE;
+    a.split   = pl.split;
+    a.nfull   = (int)pl.nfull;
+    a.part    = pl.split > 1 ? a.split_ws : nullptr;
+    a.cluster = pl.cluster;
+    a.units   = (int)units;
     gemm_fn_register(reinterpret_cast<const void *>(kern));
-    kern<<<grid, 256, SM::BYTES, stream>>>(a);
-    HEFF_LAUNCH_CHECK();
-    count_launches(sp.split > 1 ? 2 : 1);
-    if(sp.split > 1) {
-        const dim3 rgrid((unsigned)(tiles - sp.nfull), (unsigned)(SplitReduce<CPLX>::EPT / SplitReduce<CPLX>::EPB));
-        gemm_fn_register(reinterpret_cast<const void *>(gemm_split_reduce_kernel<CPLX>));
-        gemm_split_reduce_kernel<CPLX><<<rgrid, 256, 0, stream>>>(a);
+    if(pl.cluster > 1) {
+        cudaLaunchConfig_t  lc = {};
+        cudaLaunchAttribute at[1];
+        at[0].id               = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)pl.cluster;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        lc.gridDim             = dim3((unsigned)units);
+        lc.blockDim            = dim3(G::THREADS);
+        lc.dynamicSmemBytes    = SM::BYTES;
+        lc.stream              = stream;
+        lc.attrs               = at;
+        lc.numAttrs            = 1;
+        HEFF_CUDA(cudaLaunchKernelEx(&lc, kern, (const GemmArgs)a));
+    } else {
+        const int64_t slots = (int64_t)device_sm_count() * per_sm;
+        kern<<<dim3((unsigned)(units < slots ? units : slots)), G::THREADS, SM::BYTES, stream>>>(a);
+        HEFF_LAUNCH_CHECK();
+    }
+    count_launches(pl.split > 1 ? 2 : 1);
+    if(pl.split > 1) {
+        using SR = SplitReduce<CPLX, CFG>;
+        const dim3 rgrid((unsigned)(tiles - pl.nfull), (unsigned)(SR::EPT / SR::EPB));
+        gemm_fn_register(reinterpret_cast<const void *>(gemm_split_reduce_kernel<CPLX, CFG>));
+        gemm_split_reduce_kernel<CPLX, CFG><<<rgrid, G::THREADS, 0, stream>>>(a);
         HEFF_LAUNCH_CHECK();
     }
     return HEFF_OK;
 }
 
+template<bool CPLX, int CFG, int VEC>
+static int launch_ops(bool ta, bool tb, const GemmArgs &a, const GemmPlan &pl, cudaStream_t s) {
+    if(ta && tb) return HEFF_BAD_ARG;  // no caller forms A^T B^T
+    if(ta) return launch_gemm<CPLX, CFG, true, false, VEC>(a, pl, s);
+    if(tb) return launch_gemm<CPLX, CFG, false, true, VEC>(a, pl, s);
+    return launch_gemm<CPLX, CFG, false, false, VEC>(a, pl, s);
+}
+
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
-template<>
-int gemm_f64<false>(bool ta, bool tb, bool cja, const GemmArgs &a, cudaStream_t s) {
-    (void)cja;
-    if(a.M <= 0 || a.N <= 0 || a.batch <= 0) return HEFF_OK;
-    if(a.K <= 0) return HEFF_BAD_ARG;  // callers never form empty contractions
-    if(a.batch > 65535 || cdiv(a.N, GemmTile<false>::BN) > 65535) return HEFF_BAD_SHAPE;
-    // 16-byte copies need: 16B-aligned bases, even leading dims / batch strides, even contiguous extent.
-    const bool v2 = aligned16(a.A) && aligned16(a.B) && (a.lda % 2 == 0) && (a.ldb % 2 == 0) && (a.sA % 2 == 0) && (a.sB % 2 == 0) &&
-                    ((ta ? a.K : a.M) % 2 == 0) && ((tb ? a.N : a.K) % 2 == 0);
-    if(v2) {
-        if(!ta && !tb) return launch_gemm<false, false, false, false, 2>(a, s);
-        if(ta && !tb) return launch_gemm<false, true, false, false, 2>(a, s);
-        if(!ta && tb) return launch_gemm<false, false, true, false, 2>(a, s);
-        return launch_gemm<false, true, true, false, 2>(a, s);
-    }
-    if(!ta && !tb) return launch_gemm<false, false, false, false, 1>(a, s);
-    if(ta && !tb) return launch_gemm<false, true, false, false, 1>(a, s);
-    if(!ta && tb) return launch_gemm<false, false, true, false, 1>(a, s);
-    return launch_gemm<false, true, true, false, 1>(a, s);
+template<bool CPLX, int VEC>
+static int launch_plan(bool ta, bool tb, const GemmArgs &a, const GemmPlan &pl, cudaStream_t s) {
+    if(pl.cfg == 0) return launch_ops<CPLX, 0, VEC>(ta, tb, a, pl, s);
+    if(pl.cfg == 1) return launch_ops<CPLX, 1, VEC>(ta, tb, a, pl, s);
+    if constexpr(!CPLX) return launch_ops<CPLX, 2, VEC>(ta, tb, a, pl, s);
+    return HEFF_BAD_ARG;
 }
 
 template<>
-int gemm_f64<true>(bool ta, bool tb, bool cja, const GemmArgs &a, cudaStream_t s) {
+int gemm_f64<false>(bool ta, bool tb, const GemmArgs &a, cudaStream_t s) {
+    if(a.M <= 0 || a.N <= 0 || a.batch <= 0) return HEFF_OK;
+    if(a.K <= 0) return HEFF_BAD_ARG;  // callers never form empty contractions
+    // 16-byte copies need: 16B-aligned bases, even leading dims / batch strides, even contiguous extent.
+    const bool v2 = aligned16(a.A) && aligned16(a.B) && (a.lda % 2 == 0) && (a.ldb % 2 == 0) && (a.sA % 2 == 0) && (a.sB % 2 == 0) &&
+                    ((ta ? a.K : a.M) % 2 == 0) && ((tb ? a.N : a.K) % 2 == 0);
+    const GemmPlan pl = gemm_pick<false>(a);
+    return v2 ? launch_plan<false, 2>(ta, tb, a, pl, s) : launch_plan<false, 1>(ta, tb, a, pl, s);
+}
+
+template<>
+int gemm_f64<true>(bool ta, bool tb, const GemmArgs &a, cudaStream_t s) {
     if(a.M <= 0 || a.N <= 0 || a.batch <= 0) return HEFF_OK;
     if(a.K <= 0) return HEFF_BAD_ARG;
-    if(a.batch > 65535 || cdiv(a.N, GemmTile<true>::BN) > 65535) return HEFF_BAD_SHAPE;
     if(!aligned16(a.A) || !aligned16(a.B)) return HEFF_BAD_ARG;  // complex128 buffers are always 16-byte aligned
-    if(cja) {
-        if(!ta && !tb) return launch_gemm<true, false, false, true, 1>(a, s);
-        if(ta && !tb) return launch_gemm<true, true, false, true, 1>(a, s);
-        if(!ta && tb) return launch_gemm<true, false, true, true, 1>(a, s);
-        return launch_gemm<true, true, true, true, 1>(a, s);
-    }
-    if(!ta && !tb) return launch_gemm<true, false, false, false, 1>(a, s);
-    if(ta && !tb) return launch_gemm<true, true, false, false, 1>(a, s);
-    if(!ta && tb) return launch_gemm<true, false, true, false, 1>(a, s);
-    return launch_gemm<true, true, true, false, 1>(a, s);
+    return launch_plan<true, 1>(ta, tb, a, gemm_pick<true>(a), s);
 }
 
 }  // namespace heff

@@ -178,7 +178,7 @@ int matvec_fp64(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename
     g1.beta  = make_double2(0.0, 0.0);
     g1.split_ws       = ws.split_ws;
     g1.split_ws_bytes = ws.split_bytes;
-    HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, false, g1, s));
+    HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, g1, s));
     if(ev) HEFF_CUDA(cudaEventRecord(ev[2], s));
     HEFF_TRY(launch_mix<CPLX>(d, ws.T1, ws.T2, W, s));
     if(ev) HEFF_CUDA(cudaEventRecord(ev[3], s));
@@ -197,7 +197,7 @@ int matvec_fp64(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename
     g2.beta  = make_double2(0.0, 0.0);
     g2.split_ws       = ws.split_ws;
     g2.split_ws_bytes = ws.split_bytes;
-    HEFF_TRY(gemm_f64<CPLX>(false, false, false, g2, s));
+    HEFF_TRY(gemm_f64<CPLX>(false, false, g2, s));
     if(ev) HEFF_CUDA(cudaEventRecord(ev[4], s));
     return HEFF_OK;
 }
@@ -224,7 +224,7 @@ int matvec_left_stages(const MatvecDims &d, const typename Scalar<CPLX>::T *x, c
     g1.ldc   = d.cL * d.DL;
     g1.alpha = make_double2(alpha, 0.0);
     g1.beta  = make_double2(0.0, 0.0);
-    HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, false, g1, s));
+    HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, g1, s));
     return launch_mix<CPLX>(d, T1, out, W, s);
 }
 
@@ -265,7 +265,7 @@ int matvec_fp64_host(const MatvecDims &d, const typename Scalar<CPLX>::T *xh, ty
         g1.M = (int)(d.cL * d.DL), g1.N = (int)(d.S * (b1 - b0)), g1.K = (int)d.cL, g1.batch = 1;
         g1.A = L, g1.lda = d.cL, g1.B = ws.xp + o0, g1.ldb = d.cL, g1.C = ws.T1 + d.cL * d.DL * d.S * b0, g1.ldc = d.cL * d.DL;
         g1.alpha = make_double2(1.0, 0.0), g1.beta = make_double2(0.0, 0.0);
-        HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, false, g1, s));
+        HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, g1, s));
         HEFF_TRY(launch_mix<CPLX>(d, ws.T1, ws.T2, W, s, b0, b1 - b0));
     }
     // every mix (both streams) before any GEMM 2 slab
@@ -282,7 +282,7 @@ int matvec_fp64_host(const MatvecDims &d, const typename Scalar<CPLX>::T *xh, ty
         g2.M = (int)(d.S * d.cL), g2.N = (int)(b1 - b0), g2.K = (int)(d.cR * d.DR), g2.batch = 1;
         g2.A = ws.T2, g2.lda = d.S * d.cL, g2.B = Rp + d.cR * d.DR * b0, g2.ldb = d.cR * d.DR, g2.C = dy + colx * b0, g2.ldc = d.S * d.cL;
         g2.alpha = make_double2(1.0, 0.0), g2.beta = make_double2(0.0, 0.0);
-        HEFF_TRY(gemm_f64<CPLX>(false, false, false, g2, s));
+        HEFF_TRY(gemm_f64<CPLX>(false, false, g2, s));
         HEFF_CUDA(cudaEventRecord(hp.ev[HostPipe::MAXS + 3 + c], s));
         HEFF_CUDA(cudaStreamWaitEvent(hp.copy, hp.ev[HostPipe::MAXS + 3 + c], 0));
         HEFF_CUDA(cudaMemcpyAsync(yh + colx * b0, dy + colx * b0, sizeof(T) * colx * (b1 - b0), cudaMemcpyDeviceToHost, hp.copy));

@@ -116,7 +116,7 @@ int matvec_multi(const MultiDims &md, const typename Scalar<CPLX>::T *x, typenam
     g1.M = (int)(cL * D0), g1.N = (int)(S * cR), g1.K = (int)cL, g1.batch = 1;
     g1.A = L, g1.lda = cL, g1.B = xp, g1.ldb = cL, g1.C = buf[0], g1.ldc = cL * D0;
     g1.alpha = make_double2(1.0, 0.0), g1.beta = make_double2(0.0, 0.0);
-    HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, false, g1, s));
+    HEFF_TRY(gemm_f64<CPLX>(/*ta=*/true, /*tb=*/false, g1, s));
     int64_t P = 1;
     int     cur = 0;
     for(int i = 0; i < md.nmpo; i++) {
@@ -137,7 +137,7 @@ int matvec_multi(const MultiDims &md, const typename Scalar<CPLX>::T *x, typenam
     g2.M = (int)(S * cL), g2.N = (int)cR, g2.K = (int)(cR * DK), g2.batch = 1;
     g2.A = buf[cur], g2.lda = S * cL, g2.B = Rp, g2.ldb = cR * DK, g2.C = y, g2.ldc = S * cL;
     g2.alpha = make_double2(1.0, 0.0), g2.beta = make_double2(0.0, 0.0);
-    return gemm_f64<CPLX>(false, false, false, g2, s);
+    return gemm_f64<CPLX>(false, false, g2, s);
 }
 
 template int matvec_multi<false>(const MultiDims &, const double *, double *, const double *, const double *, const double *const *, double *,
