@@ -39,6 +39,7 @@ constexpr int MD_G = 8;
 template<class T>
 __global__ void __launch_bounds__(256) multi_dot_partial(const T *__restrict__ V, int64_t ldv, int64_t n, int k, const T *__restrict__ t,
                                                         double *__restrict__ partials) {
+    grid_wait();
     constexpr bool CPLX = sizeof(T) == 16;
     __shared__ double sre[8][MD_G], sim[8][MD_G];
     const int         lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(256) multi_dot_partial(const T *__restrict__ V
 // One block per column: fixed-order tree reduction of the nb partial sums.
 template<class T>
 __global__ void __launch_bounds__(256) multi_dot_final(const double *__restrict__ partials, int nb, int k, T *__restrict__ h) {
+    grid_wait();
     __shared__ double sa[256], sb[256];
     const int         j = blockIdx.x;
     double            a = 0, b = 0;
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(256) multi_dot_final(const double *__restrict_
 
 template<class T>
 __global__ void multi_axpy_kernel(const T *__restrict__ V, int64_t ldv, int64_t n, int k, const T *__restrict__ h, double alpha, T *__restrict__ t) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char hsm[];
     T *sh = reinterpret_cast<T *>(hsm);
     for(int j = threadIdx.x; j < k; j += blockDim.x) sh[j] = h[j];
@@ -123,6 +126,7 @@ __global__ void multi_axpy_kernel(const T *__restrict__ V, int64_t ldv, int64_t 
 
 template<class T>
 __global__ void combine_kernel(const T *__restrict__ V, int64_t ldv, int64_t n, int k, const T *__restrict__ c, T *__restrict__ x) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char csm[];
     T *sc = reinterpret_cast<T *>(csm);
     for(int j = threadIdx.x; j < k; j += blockDim.x) sc[j] = c[j];
@@ -136,12 +140,14 @@ __global__ void combine_kernel(const T *__restrict__ V, int64_t ldv, int64_t n, 
 
 template<class T>
 __global__ void scale_kernel(T *__restrict__ x, int64_t n, const double *__restrict__ a, bool inv_sqrt) {
+    grid_wait();
     const double v = inv_sqrt ? (a[0] > 0 ? rsqrt(a[0]) : 0.0) : a[0];
     for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] = VOps<T>::scale(x[i], v);
 }
 
 template<class T>
 __global__ void residual_kernel(const T *__restrict__ ax, const T *__restrict__ x, double theta, T *__restrict__ r, int64_t n) {
+    grid_wait();
     for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         r[i] = VOps<T>::addscaled(ax[i], -theta, x[i]);
 }
@@ -158,10 +164,8 @@ int multi_dot(const typename Scalar<CPLX>::T *V, int64_t ldv, int64_t n, int k, 
     if(k <= 0) return HEFF_OK;
     if(k > MD_MAXK) return HEFF_BAD_ARG;
     const int nb = (int)std::min<int64_t>(std::min<int64_t>(MD_BLOCKS, 4 * (int64_t)device_sm_count()), std::max<int64_t>(1, (n + 255) / 256));
-    multi_dot_partial<T><<<nb, 256, 0, s>>>(V, ldv, n, k, t, partials);
-    HEFF_LAUNCH_CHECK();
-    multi_dot_final<T><<<k, 256, 0, s>>>(partials, nb, k, h);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(multi_dot_partial<T>, nb, 256, 0, s, V, ldv, n, k, t, partials)));
+    HEFF_CUDA((launch_chained(multi_dot_final<T>, k, 256, 0, s, partials, nb, k, h)));
     return HEFF_OK;
 }
 
@@ -170,8 +174,7 @@ int multi_axpy(const typename Scalar<CPLX>::T *V, int64_t ldv, int64_t n, int k,
                typename Scalar<CPLX>::T *t, cudaStream_t s) {
     using T = typename Scalar<CPLX>::T;
     if(k <= 0) return HEFF_OK;
-    multi_axpy_kernel<T><<<grid_for(n), 256, sizeof(T) * k, s>>>(V, ldv, n, k, h, alpha, t);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(multi_axpy_kernel<T>, grid_for(n), 256, sizeof(T) * k, s, V, ldv, n, k, h, alpha, t)));
     return HEFF_OK;
 }
 
@@ -179,23 +182,20 @@ template<bool CPLX>
 int combine(const typename Scalar<CPLX>::T *V, int64_t ldv, int64_t n, int k, const typename Scalar<CPLX>::T *c, typename Scalar<CPLX>::T *x,
             cudaStream_t s) {
     using T = typename Scalar<CPLX>::T;
-    combine_kernel<T><<<grid_for(n), 256, sizeof(T) * std::max(k, 1), s>>>(V, ldv, n, k, c, x);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(combine_kernel<T>, grid_for(n), 256, sizeof(T) * std::max(k, 1), s, V, ldv, n, k, c, x)));
     return HEFF_OK;
 }
 
 template<bool CPLX>
 int scale_dev(typename Scalar<CPLX>::T *x, int64_t n, const double *a, bool inv_sqrt, cudaStream_t s) {
-    scale_kernel<typename Scalar<CPLX>::T><<<grid_for(n), 256, 0, s>>>(x, n, a, inv_sqrt);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(scale_kernel<typename Scalar<CPLX>::T>, grid_for(n), 256, 0, s, x, n, a, inv_sqrt)));
     return HEFF_OK;
 }
 
 template<bool CPLX>
 int residual(const typename Scalar<CPLX>::T *ax, const typename Scalar<CPLX>::T *x, double theta, typename Scalar<CPLX>::T *r, int64_t n,
              cudaStream_t s) {
-    residual_kernel<typename Scalar<CPLX>::T><<<grid_for(n), 256, 0, s>>>(ax, x, theta, r, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(residual_kernel<typename Scalar<CPLX>::T>, grid_for(n), 256, 0, s, ax, x, theta, r, n)));
     return HEFF_OK;
 }
 
@@ -221,6 +221,7 @@ template<class T>
 __global__ void __launch_bounds__(256) orth_dot_kernel(const T *__restrict__ V, int64_t ldv, int64_t n, int k, const T *__restrict__ t,
                                                       double *__restrict__ partials, unsigned *__restrict__ counter, double *__restrict__ st,
                                                       T *__restrict__ hres, int pass) {
+    grid_wait();
     constexpr bool CPLX = sizeof(T) == 16;
     if(pass == 1 && st[1] == 0.0) return;  // uniform over the grid
     __shared__ double sre[8][MD_G], sim[8][MD_G];
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(256) orth_dot_kernel(const T *__restrict__ V, 
 template<class T>
 __global__ void orth_axpy_kernel(const T *__restrict__ V, int64_t ldv, int64_t n, int k, const T *in, T *out, const double *__restrict__ st,
                                  int pass) {
+    grid_wait();
     if(pass == 1 && st[1] == 0.0) return;
     extern __shared__ __align__(16) unsigned char osm[];
     T            *sh   = reinterpret_cast<T *>(osm);
@@ -353,6 +355,7 @@ template<bool CPLX, int KM, int MODE>
 __global__ void __launch_bounds__(256, 1) orth_fast_kernel(const double2 *V, int64_t ldu, int64_t nu, int k, const double2 *in, double2 *out,
                                                            double *__restrict__ partials, unsigned *__restrict__ counter, double *__restrict__ st,
                                                            typename Scalar<CPLX>::T *__restrict__ hres) {
+    grid_wait();
     using T = typename Scalar<CPLX>::T;
     if(MODE == 2 && st[1] == 0.0) return;  // uniform over the grid
     __shared__ double sre[8][KM + 1], sim[8][KM + 1];
@@ -479,12 +482,9 @@ template<bool CPLX, int KM>
 static int orth_fast(const double2 *V, int64_t ldu, int64_t nu, int k, const double2 *w, double2 *v, double *partials, unsigned *counter, double *st,
                      typename Scalar<CPLX>::T *hres, cudaStream_t s) {
     const int nb = (int)std::min<int64_t>(std::min<int64_t>(MD_BLOCKS, 4 * (int64_t)device_sm_count()), std::max<int64_t>(1, (nu + 255) / 256));
-    orth_fast_kernel<CPLX, KM, 0><<<nb, 256, 0, s>>>(V, ldu, nu, k, w, nullptr, partials, counter, st, hres);
-    HEFF_LAUNCH_CHECK();
-    orth_fast_kernel<CPLX, KM, 1><<<nb, 256, 0, s>>>(V, ldu, nu, k, w, v, partials, counter, st, hres);
-    HEFF_LAUNCH_CHECK();
-    orth_fast_kernel<CPLX, KM, 2><<<nb, 256, 0, s>>>(V, ldu, nu, k, v, v, partials, counter, st, hres);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(orth_fast_kernel<CPLX, KM, 0>, nb, 256, 0, s, V, ldu, nu, k, w, nullptr, partials, counter, st, hres)));
+    HEFF_CUDA((launch_chained(orth_fast_kernel<CPLX, KM, 1>, nb, 256, 0, s, V, ldu, nu, k, w, v, partials, counter, st, hres)));
+    HEFF_CUDA((launch_chained(orth_fast_kernel<CPLX, KM, 2>, nb, 256, 0, s, V, ldu, nu, k, v, v, partials, counter, st, hres)));
     return HEFF_OK;
 }
 
@@ -505,14 +505,10 @@ int orth_cgs2(const typename Scalar<CPLX>::T *V, int64_t ldv, int64_t n, int k, 
         return orth_fast<CPLX, 24>(V2, ldu, nu, k, w2, v2, partials, counter, st, hres, s);
     }
     const int nb = (int)std::min<int64_t>(std::min<int64_t>(MD_BLOCKS, 4 * (int64_t)device_sm_count()), std::max<int64_t>(1, (n + 255) / 256));
-    orth_dot_kernel<T><<<nb, 256, 0, s>>>(V, ldv, n, k, w, partials, counter, st, hres, 0);
-    HEFF_LAUNCH_CHECK();
-    orth_axpy_kernel<T><<<grid_for(n), 256, sizeof(T) * k, s>>>(V, ldv, n, k, w, v, st, 0);
-    HEFF_LAUNCH_CHECK();
-    orth_dot_kernel<T><<<nb, 256, 0, s>>>(V, ldv, n, k, v, partials, counter, st, hres, 1);
-    HEFF_LAUNCH_CHECK();
-    orth_axpy_kernel<T><<<grid_for(n), 256, sizeof(T) * k, s>>>(V, ldv, n, k, v, v, st, 1);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(orth_dot_kernel<T>, nb, 256, 0, s, V, ldv, n, k, w, partials, counter, st, hres, 0)));
+    HEFF_CUDA((launch_chained(orth_axpy_kernel<T>, grid_for(n), 256, sizeof(T) * k, s, V, ldv, n, k, w, v, st, 0)));
+    HEFF_CUDA((launch_chained(orth_dot_kernel<T>, nb, 256, 0, s, V, ldv, n, k, v, partials, counter, st, hres, 1)));
+    HEFF_CUDA((launch_chained(orth_axpy_kernel<T>, grid_for(n), 256, sizeof(T) * k, s, V, ldv, n, k, v, v, st, 1)));
     return HEFF_OK;
 }
 
@@ -565,6 +561,7 @@ __device__ bool grid_reduce_last(double (&v)[NV], double *__restrict__ partials,
 template<class T>
 __global__ void cg_init_kernel(T *__restrict__ d, T *__restrict__ r, T *__restrict__ p, const T *__restrict__ r0, int64_t n, double *__restrict__ cs,
                                double rho0, double theta, double tol2) {
+    grid_wait();
     for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const T v = VOps<T>::scale(r0[i], -1.0);
         d[i]      = VOps<T>::zero();
@@ -587,6 +584,7 @@ __device__ __forceinline__ void cj_acc(double &re, double &im, double2 a, double
 template<class T>
 __global__ void __launch_bounds__(256) cg_a_kernel(const T *__restrict__ z, const T *__restrict__ p, const T *__restrict__ u, T *__restrict__ q,
                                                   int64_t n, double *__restrict__ cs, double *__restrict__ partials, unsigned *__restrict__ counter) {
+    grid_wait();
     if(cs[CG_DONE] != 0.0) return;
     const double theta = cs[CG_THETA];
     double       v[6]  = {0, 0, 0, 0, 0, 0};  // u^H q, p^H q, p^H u (re, im)
@@ -617,6 +615,7 @@ template<class T>
 __global__ void __launch_bounds__(256) cg_b_kernel(const T *__restrict__ q, const T *__restrict__ u, const T *__restrict__ p, T *__restrict__ d,
                                                   T *__restrict__ r, int64_t n, double *__restrict__ cs, double *__restrict__ partials,
                                                   unsigned *__restrict__ counter) {
+    grid_wait();
     if(cs[CG_DONE] != 0.0) return;
     const double alpha = cs[CG_ALPHA];
     const T      c     = VOps<T>::make(cs[CG_CRE], cs[CG_CIM]);
@@ -643,6 +642,7 @@ __global__ void __launch_bounds__(256) cg_b_kernel(const T *__restrict__ q, cons
 // p = r + beta p
 template<class T>
 __global__ void cg_c_kernel(const T *__restrict__ r, T *__restrict__ p, int64_t n, const double *__restrict__ cs) {
+    grid_wait();
     if(cs[CG_DONE] != 0.0) return;
     const double beta = cs[CG_BETA];
     for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -652,8 +652,7 @@ __global__ void cg_c_kernel(const T *__restrict__ r, T *__restrict__ p, int64_t 
 template<bool CPLX>
 int cg_init(typename Scalar<CPLX>::T *d, typename Scalar<CPLX>::T *r, typename Scalar<CPLX>::T *p, const typename Scalar<CPLX>::T *r0, int64_t n,
             double *cs, double rho0, double theta, double tol2, cudaStream_t s) {
-    cg_init_kernel<typename Scalar<CPLX>::T><<<grid_for(n), 256, 0, s>>>(d, r, p, r0, n, cs, rho0, theta, tol2);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(cg_init_kernel<typename Scalar<CPLX>::T>, grid_for(n), 256, 0, s, d, r, p, r0, n, cs, rho0, theta, tol2)));
     return HEFF_OK;
 }
 
@@ -662,12 +661,9 @@ int cg_step(const typename Scalar<CPLX>::T *z, typename Scalar<CPLX>::T *p, cons
             typename Scalar<CPLX>::T *d, typename Scalar<CPLX>::T *r, int64_t n, double *cs, double *partials, unsigned *counter, cudaStream_t s) {
     using T      = typename Scalar<CPLX>::T;
     const int nb = (int)std::min<int64_t>(std::min<int64_t>(MD_BLOCKS, 4 * (int64_t)device_sm_count()), std::max<int64_t>(1, (n + 255) / 256));
-    cg_a_kernel<T><<<nb, 256, 0, s>>>(z, p, u, q, n, cs, partials, counter);
-    HEFF_LAUNCH_CHECK();
-    cg_b_kernel<T><<<nb, 256, 0, s>>>(q, u, p, d, r, n, cs, partials, counter);
-    HEFF_LAUNCH_CHECK();
-    cg_c_kernel<T><<<grid_for(n), 256, 0, s>>>(r, p, n, cs);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(cg_a_kernel<T>, nb, 256, 0, s, z, p, u, q, n, cs, partials, counter)));
+    HEFF_CUDA((launch_chained(cg_b_kernel<T>, nb, 256, 0, s, q, u, p, d, r, n, cs, partials, counter)));
+    HEFF_CUDA((launch_chained(cg_c_kernel<T>, grid_for(n), 256, 0, s, r, p, n, cs)));
     return HEFF_OK;
 }
 

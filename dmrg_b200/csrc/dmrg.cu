@@ -110,6 +110,7 @@ static void ising_site_mpo2(std::vector<double> &W2, int64_t wd[4], int i, int L
 
 // C[(s1 + d a) + d ca (s2 + d b)] -> theta[(s1 + d s2) + d^2 (a + ca b)]
 __global__ void merge_layout_kernel(const double *__restrict__ C, double *__restrict__ th, int64_t d, int64_t ca, int64_t cb) {
+    grid_wait();
     const int64_t tot = d * d * ca * cb;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = e % (d * d), r = e / (d * d), a = r % ca, b = r / ca;
@@ -119,6 +120,7 @@ __global__ void merge_layout_kernel(const double *__restrict__ C, double *__rest
 }
 // M2p[c + cc (s2 + d b)] = M2[s2 + d (c + cc b)]
 __global__ void perm_sc_kernel(const double *__restrict__ M, double *__restrict__ P, int64_t d, int64_t cc, int64_t cb) {
+    grid_wait();
     const int64_t tot = d * cc * cb;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t c = e % cc, r = e / cc, s2 = r % d, b = r / d;
@@ -127,6 +129,7 @@ __global__ void perm_sc_kernel(const double *__restrict__ M, double *__restrict_
 }
 // X[s, a, k] *= S[k] (which = 0) or X[s, k, b] *= S[k] (which = 1)
 __global__ void scale_bond_kernel(double *__restrict__ X, const double *__restrict__ S, int64_t d, int64_t n1, int64_t n2, int which) {
+    grid_wait();
     const int64_t tot = d * n1 * n2;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = e / d, i1 = r % n1, i2 = r / n1;
@@ -294,15 +297,13 @@ static int dmrg_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, DmrgW
                 const int     i  = dir == 0 ? step : (L - 2 - step);
                 const int64_t ca = chi[i], cc = chi[i + 1], cb = chi[i + 2];
                 // theta = M_i M_{i+1}
-                perm_sc_kernel<<<g1(d * cc * cb), 256, 0, s>>>(ws.M[i + 1], ws.P2, d, cc, cb);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(perm_sc_kernel, g1(d * cc * cb), 256, 0, s, ws.M[i + 1], ws.P2, d, cc, cb)));
                 GemmArgs g{};
                 g.M = (int)(d * ca), g.N = (int)(d * cb), g.K = (int)cc, g.batch = 1;
                 g.A = ws.M[i], g.lda = d * ca, g.B = ws.P2, g.ldb = cc, g.C = ws.Cbuf, g.ldc = d * ca;
                 g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
                 HEFF_TRY(gemm_f64<false>(false, false, g, s));
-                merge_layout_kernel<<<g1(d * d * ca * cb), 256, 0, s>>>(ws.Cbuf, ws.theta, d, ca, cb);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(merge_layout_kernel, g1(d * d * ca * cb), 256, 0, s, ws.Cbuf, ws.theta, d, ca, cb)));
                 // eigensolve on the rebound operator
                 auto          te0   = now();
                 const void   *mp[2] = {Wh[i].data(), Wh[i + 1].data()};
@@ -343,15 +344,13 @@ static int dmrg_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, DmrgW
                 auto tv0   = now();
                 if(dir == 0) {
                     HEFF_CUDA(cudaMemcpyAsync(ws.M[i], ws.U, sizeof(double) * d * ca * k, cudaMemcpyDeviceToDevice, s));
-                    scale_bond_kernel<<<g1(d * k * cb), 256, 0, s>>>(ws.V, ws.S, d, k, cb, 1);
-                    HEFF_LAUNCH_CHECK();
+                    HEFF_CUDA((launch_chained(scale_bond_kernel, g1(d * k * cb), 256, 0, s, ws.V, ws.S, d, k, cb, 1)));
                     HEFF_CUDA(cudaMemcpyAsync(ws.M[i + 1], ws.V, sizeof(double) * d * k * cb, cudaMemcpyDeviceToDevice, s));
                     const int64_t ed[3] = {ca, ca, wd[i][0]}, mdd[3] = {d, ca, k};
                     HEFF_TRY(env_update_d(0, ws.Lenv[i + 1], ws.Lenv[i], ed, ws.M[i], mdd, ws.W[i], wd[i].data(), ws.scr, s, ws.op->split_ws, ws.op->split_bytes));
                 } else {
                     HEFF_CUDA(cudaMemcpyAsync(ws.M[i + 1], ws.V, sizeof(double) * d * k * cb, cudaMemcpyDeviceToDevice, s));
-                    scale_bond_kernel<<<g1(d * ca * k), 256, 0, s>>>(ws.U, ws.S, d, ca, k, 0);
-                    HEFF_LAUNCH_CHECK();
+                    HEFF_CUDA((launch_chained(scale_bond_kernel, g1(d * ca * k), 256, 0, s, ws.U, ws.S, d, ca, k, 0)));
                     HEFF_CUDA(cudaMemcpyAsync(ws.M[i], ws.U, sizeof(double) * d * ca * k, cudaMemcpyDeviceToDevice, s));
                     const int64_t ed[3] = {cb, cb, wd[i + 1][1]}, mdd[3] = {d, k, cb};
                     HEFF_TRY(env_update_d(1, ws.Renv[i], ws.Renv[i + 1], ed, ws.M[i + 1], mdd, ws.W[i + 1], wd[i + 1].data(), ws.scr, s, ws.op->split_ws, ws.op->split_bytes));
@@ -381,15 +380,13 @@ static int dmrg_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, DmrgW
             HEFF_TRY(env_update_d(1, ws.Lenv[i], ws.Lenv[i + 1], ed, ws.M[i + 1], mdd, ws.W[i + 1], w3[i + 1].data(), ws.scr, s, ws.op->split_ws, ws.op->split_bytes));
         }
         const int64_t ca = chi[0], cc = chi[1], cb = chi[2];
-        perm_sc_kernel<<<g1(d * cc * cb), 256, 0, s>>>(ws.M[1], ws.P2, d, cc, cb);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(perm_sc_kernel, g1(d * cc * cb), 256, 0, s, ws.M[1], ws.P2, d, cc, cb)));
         GemmArgs g{};
         g.M = (int)(d * ca), g.N = (int)(d * cb), g.K = (int)cc, g.batch = 1;
         g.A = ws.M[0], g.lda = d * ca, g.B = ws.P2, g.ldb = cc, g.C = ws.Cbuf, g.ldc = d * ca;
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
         HEFF_TRY(gemm_f64<false>(false, false, g, s));
-        merge_layout_kernel<<<g1(d * d * ca * cb), 256, 0, s>>>(ws.Cbuf, ws.theta, d, ca, cb);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(merge_layout_kernel, g1(d * d * ca * cb), 256, 0, s, ws.Cbuf, ws.theta, d, ca, cb)));
         // Lenv[0] still holds the trivial left edge (1)
         const void   *mp[2] = {W3h[0].data(), W3h[1].data()};
         int64_t       mdims[8];
@@ -441,6 +438,7 @@ static int dmrg_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, DmrgW
 // expansion term P[s + d (b + cb (a + c m))]
 __global__ void ex_rows_R_kernel(const double *__restrict__ B, const double *__restrict__ P, double *__restrict__ X, int64_t d, int64_t c, int64_t DL,
                                  int64_t cb) {
+    grid_wait();
     const int64_t c2 = c * (1 + DL), tot = c2 * d * cb;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a2 = e % c2, col = e / c2, s = col % d, b = col / d;
@@ -449,6 +447,7 @@ __global__ void ex_rows_R_kernel(const double *__restrict__ B, const double *__r
 }
 // site tensor [s, a, b] -> its left-bond rows X[a + c (s + d b)]
 __global__ void site_rows_kernel(const double *__restrict__ M, double *__restrict__ X, int64_t d, int64_t c, int64_t cb) {
+    grid_wait();
     const int64_t tot = d * c * cb;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = e % c, col = e / c, s = col % d, b = col / d;
@@ -457,6 +456,7 @@ __global__ void site_rows_kernel(const double *__restrict__ M, double *__restric
 }
 // rows X[a + ldx (s + d b)] (a < c) -> site tensor M[s + d (a + c b)]
 __global__ void rows_site_kernel(const double *__restrict__ X, int64_t ldx, double *__restrict__ M, int64_t d, int64_t c, int64_t cb) {
+    grid_wait();
     const int64_t tot = d * c * cb;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = e % d, r = e / d, a = r % c, b = r / c;
@@ -465,6 +465,7 @@ __global__ void rows_site_kernel(const double *__restrict__ X, int64_t ldx, doub
 }
 // which 0: X[r + ld k] *= S[k] (columns); which 1: X[k + ld j] *= S[k] (rows); rows x cols of X
 __global__ void scale_mat_kernel(double *__restrict__ X, int64_t ld, int64_t rows, int64_t cols, const double *__restrict__ S, int which) {
+    grid_wait();
     const int64_t tot = rows * cols;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = e % rows, c = e / rows;
@@ -473,6 +474,7 @@ __global__ void scale_mat_kernel(double *__restrict__ X, int64_t ld, int64_t row
 }
 // Y[j + ldy i] = X[i + ldx j] for i < rows, j < cols
 __global__ void transpose_kernel(const double *__restrict__ X, int64_t ldx, int64_t rows, int64_t cols, double *__restrict__ Y, int64_t ldy) {
+    grid_wait();
     const int64_t tot = rows * cols;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = e % rows, j = e / rows;
@@ -494,14 +496,11 @@ static int gemm_nn(const double *A, int64_t lda, const double *B, int64_t ldb, d
 static int svd_oriented(DmrgWorkspace &ws, const double *A, int64_t lda, int64_t m, int64_t n, int64_t rank_max, double trunc, double *U, double *S,
                         double *VT, int64_t *k, double *err, cudaStream_t s) {
     if(m >= n) return svd_truncated(A, lda, m, n, rank_max, trunc, U, S, VT, k, err, ws.escr, nullptr, s);
-    transpose_kernel<<<g1(m * n), 256, 0, s>>>(A, lda, m, n, ws.eT, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(transpose_kernel, g1(m * n), 256, 0, s, A, lda, m, n, ws.eT, n)));
     HEFF_TRY(svd_truncated(ws.eT, n, n, m, rank_max, trunc, ws.eY, S, ws.eZ, k, err, ws.escr, nullptr, s));
     // A^T = U' S VT'  ->  A = VT'^T S U'^T
-    transpose_kernel<<<g1(*k * m), 256, 0, s>>>(ws.eZ, *k, *k, m, U, m);
-    HEFF_LAUNCH_CHECK();
-    transpose_kernel<<<g1(n * *k), 256, 0, s>>>(ws.eY, n, n, *k, VT, *k);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(transpose_kernel, g1(*k * m), 256, 0, s, ws.eZ, *k, *k, m, U, m)));
+    HEFF_CUDA((launch_chained(transpose_kernel, g1(n * *k), 256, 0, s, ws.eY, n, n, *k, VT, *k)));
     return HEFF_OK;
 }
 
@@ -620,19 +619,16 @@ static int dmrg1_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, Dmrg
                 const int64_t ed[3] = {cb, cb, wd[i + 1][1]}, mdd[3] = {d, c, cb};
                 HEFF_TRY(expansion_term<false>(1, ws.eP, ws.Renv[i + 1], ed, ws.M[i + 1], mdd, ws.W[i + 1], wd[i + 1].data(), alpha, s));
                 const int64_t c2 = c * (1 + DL);
-                ex_rows_R_kernel<<<g1(c2 * d * cb), 256, 0, s>>>(ws.M[i + 1], ws.eP, ws.eX, d, c, DL, cb);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(ex_rows_R_kernel, g1(c2 * d * cb), 256, 0, s, ws.M[i + 1], ws.eP, ws.eX, d, c, DL, cb)));
                 const int64_t rmax = std::min(std::min(d * ca, d * cb), chi_lim);
                 int64_t       k    = 0;
                 double        te   = 0;
                 HEFF_TRY(svd_oriented(ws, ws.eX, c2, c2, d * cb, rmax, cfg.trunc_lim, ws.eU, ws.S, ws.eV, &k, &te, s));
                 // AC(i) <- AC(i) U[0:c, :] S ; B(i+1) <- V
                 HEFF_TRY(gemm_nn(ws.M[i], d * ca, ws.eU, c2, ws.Cbuf, d * ca, d * ca, k, c, s));
-                scale_mat_kernel<<<g1(d * ca * k), 256, 0, s>>>(ws.Cbuf, d * ca, d * ca, k, ws.S, 0);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(scale_mat_kernel, g1(d * ca * k), 256, 0, s, ws.Cbuf, d * ca, d * ca, k, ws.S, 0)));
                 HEFF_CUDA(cudaMemcpyAsync(ws.M[i], ws.Cbuf, sizeof(double) * d * ca * k, cudaMemcpyDeviceToDevice, s));
-                rows_site_kernel<<<g1(d * k * cb), 256, 0, s>>>(ws.eV, k, ws.M[i + 1], d, k, cb);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(rows_site_kernel, g1(d * k * cb), 256, 0, s, ws.eV, k, ws.M[i + 1], d, k, cb)));
                 chi[i + 1] = k;
                 auto tv0   = now();
                 HEFF_TRY(renv(i));
@@ -650,13 +646,10 @@ static int dmrg1_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, Dmrg
             res.trunc_err_max = std::max(res.trunc_err_max, te);
             record_mid(i + 1, sweep);
             HEFF_CUDA(cudaMemcpyAsync(ws.M[i], ws.eU, sizeof(double) * d * ca * k, cudaMemcpyDeviceToDevice, s));
-            scale_mat_kernel<<<g1(k * c), 256, 0, s>>>(ws.eV, k, k, c, ws.S, 1);
-            HEFF_LAUNCH_CHECK();
-            site_rows_kernel<<<g1(d * c * cb), 256, 0, s>>>(ws.M[i + 1], ws.eX, d, c, cb);
-            HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(scale_mat_kernel, g1(k * c), 256, 0, s, ws.eV, k, k, c, ws.S, 1)));
+            HEFF_CUDA((launch_chained(site_rows_kernel, g1(d * c * cb), 256, 0, s, ws.M[i + 1], ws.eX, d, c, cb)));
             HEFF_TRY(gemm_nn(ws.eV, k, ws.eX, c, ws.eZ, k, k, d * cb, c, s));
-            rows_site_kernel<<<g1(d * k * cb), 256, 0, s>>>(ws.eZ, k, ws.M[i + 1], d, k, cb);
-            HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(rows_site_kernel, g1(d * k * cb), 256, 0, s, ws.eZ, k, ws.M[i + 1], d, k, cb)));
             chi[i + 1] = k;
             t_svd += secs(ts1, now());
             auto tv0 = now();
@@ -679,13 +672,10 @@ static int dmrg1_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, Dmrg
                 HEFF_TRY(svd_oriented(ws, ws.eX, d * ca, d * ca, c2, rmax, cfg.trunc_lim, ws.eU, ws.S, ws.eV, &k, &te, s));
                 // A(i-1) <- U ; AC(i) <- S V[:, 0:c] AC(i)
                 HEFF_CUDA(cudaMemcpyAsync(ws.M[i - 1], ws.eU, sizeof(double) * d * ca * k, cudaMemcpyDeviceToDevice, s));
-                scale_mat_kernel<<<g1(k * c), 256, 0, s>>>(ws.eV, k, k, c, ws.S, 1);
-                HEFF_LAUNCH_CHECK();
-                site_rows_kernel<<<g1(d * c * cb), 256, 0, s>>>(ws.M[i], ws.eP, d, c, cb);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(scale_mat_kernel, g1(k * c), 256, 0, s, ws.eV, k, k, c, ws.S, 1)));
+                HEFF_CUDA((launch_chained(site_rows_kernel, g1(d * c * cb), 256, 0, s, ws.M[i], ws.eP, d, c, cb)));
                 HEFF_TRY(gemm_nn(ws.eV, k, ws.eP, c, ws.eZ, k, k, d * cb, c, s));
-                rows_site_kernel<<<g1(d * k * cb), 256, 0, s>>>(ws.eZ, k, ws.M[i], d, k, cb);
-                HEFF_LAUNCH_CHECK();
+                HEFF_CUDA((launch_chained(rows_site_kernel, g1(d * k * cb), 256, 0, s, ws.eZ, k, ws.M[i], d, k, cb)));
                 chi[i] = k;
                 auto tv0 = now();
                 HEFF_TRY(lenv(i - 1));
@@ -696,19 +686,16 @@ static int dmrg1_run_ws(const heff_dmrg_config &cfg, heff_dmrg_result &res, Dmrg
             // split AC(i) = U S B(i); AC(i-1) = A(i-1) U S
             auto          ts1 = now();
             const int64_t ca = chi[i - 1], c = chi[i], cb = chi[i + 1];
-            site_rows_kernel<<<g1(d * c * cb), 256, 0, s>>>(ws.M[i], ws.eX, d, c, cb);
-            HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(site_rows_kernel, g1(d * c * cb), 256, 0, s, ws.M[i], ws.eX, d, c, cb)));
             int64_t k  = 0;
             double  te = 0;
             HEFF_TRY(svd_oriented(ws, ws.eX, c, c, d * cb, chi_lim, cfg.trunc_lim, ws.eU, ws.S, ws.eV, &k, &te, s));
             HEFF_TRY(normalise_S(ws.S, k, hs, s));
             res.trunc_err_max = std::max(res.trunc_err_max, te);
             record_mid(i, sweep);
-            rows_site_kernel<<<g1(d * k * cb), 256, 0, s>>>(ws.eV, k, ws.M[i], d, k, cb);
-            HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(rows_site_kernel, g1(d * k * cb), 256, 0, s, ws.eV, k, ws.M[i], d, k, cb)));
             HEFF_TRY(gemm_nn(ws.M[i - 1], d * ca, ws.eU, c, ws.Cbuf, d * ca, d * ca, k, c, s));
-            scale_mat_kernel<<<g1(d * ca * k), 256, 0, s>>>(ws.Cbuf, d * ca, d * ca, k, ws.S, 0);
-            HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(scale_mat_kernel, g1(d * ca * k), 256, 0, s, ws.Cbuf, d * ca, d * ca, k, ws.S, 0)));
             HEFF_CUDA(cudaMemcpyAsync(ws.M[i - 1], ws.Cbuf, sizeof(double) * d * ca * k, cudaMemcpyDeviceToDevice, s));
             chi[i] = k;
             t_svd += secs(ts1, now());

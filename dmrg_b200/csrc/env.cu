@@ -29,6 +29,7 @@ __device__ __forceinline__ void setz(double2 &v) { v = make_double2(0.0, 0.0); }
 // Mc[a' + cL*(s' + d*b')] = conj(M[s' + d*(a' + cL*b')])
 template<class T>
 __global__ void env_prep_L(const T *__restrict__ M, T *__restrict__ Mc, int64_t d, int64_t cL, int64_t n) {
+    grid_wait();
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t ap = o % cL, r = o / cL, sp = r % d, bp = r / d;
         Mc[o]            = conj_s(M[sp + d * (ap + cL * bp)]);
@@ -37,6 +38,7 @@ __global__ void env_prep_L(const T *__restrict__ M, T *__restrict__ Mc, int64_t 
 // Mc[i] = conj(M[i]);  M2[s + d*(b + cR*a)] = M[s + d*(a + cL*b)]
 template<class T>
 __global__ void env_prep_R(const T *__restrict__ M, T *__restrict__ Mc, T *__restrict__ M2, int64_t d, int64_t cL, int64_t cR, int64_t n) {
+    grid_wait();
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         Mc[o]           = conj_s(M[o]);
         const int64_t s = o % d, r = o / d, b = r % cR, a = r / cR;
@@ -51,6 +53,7 @@ __global__ void env_prep_R(const T *__restrict__ M, T *__restrict__ Mc, T *__res
 //   L: out[n,s] = sum_{m,s'} W[m,n,s,s'] in[m,s'];   R: out[m,s] = sum_{n,s'} W[m,n,s,s'] in[n,s']
 template<class T, bool LEFT>
 __global__ void env_mix_kernel(const T *__restrict__ X, T *__restrict__ Y, const T *__restrict__ W, int d, int P, int Q, int DL, int DR) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char env_smem[];
     T        *sW = reinterpret_cast<T *>(env_smem);
     const int nW = DL * DR * d * d;
@@ -125,8 +128,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
     T            *Y   = X + pad(Dm * nM);
     const size_t  wsm = sizeof(T) * (size_t)(DL * DR * d * d);
     if(side == 0) {
-        env_prep_L<<<grid1(nM), 256, 0, s>>>(M, Mc, d, cL, nM);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(env_prep_L<T>, grid1(nM), 256, 0, s, M, Mc, d, cL, nM)));
         GemmArgs g{};
         g.M = (int)cL, g.N = (int)(d * cR), g.K = (int)cL, g.batch = (int)DL;
         g.A = E, g.lda = cL, g.sA = cL * cL;
@@ -136,8 +138,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
         if(cR > 65535) return HEFF_BAD_SHAPE;
         dim3 grid((unsigned)cdiv(cL, 128), (unsigned)cR);
-        env_mix_kernel<T, true><<<grid, 128, wsm, s>>>(X, Y, W, (int)d, (int)cL, (int)cR, (int)DL, (int)DR);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(env_mix_kernel<T, true>, grid, 128, wsm, s, X, Y, W, (int)d, (int)cL, (int)cR, (int)DL, (int)DR)));
         GemmArgs h{};
         h.M = (int)cR, h.N = (int)(cR * DR), h.K = (int)(d * cL), h.batch = 1;
         h.A = M, h.lda = d * cL, h.B = Y, h.ldb = d * cL, h.C = out, h.ldc = cR;
@@ -145,8 +146,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         h.split_ws = split_ws, h.split_ws_bytes = split_bytes;
         HEFF_TRY(gemm_f64<CPLX>(true, false, h, s));
     } else {
-        env_prep_R<<<grid1(nM), 256, 0, s>>>(M, Mc, M2, d, cL, cR, nM);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(env_prep_R<T>, grid1(nM), 256, 0, s, M, Mc, M2, d, cL, cR, nM)));
         GemmArgs g{};
         g.M = (int)cR, g.N = (int)(d * cL), g.K = (int)cR, g.batch = (int)DR;
         g.A = E, g.lda = cR, g.sA = cR * cR;
@@ -156,8 +156,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         HEFF_TRY(gemm_f64<CPLX>(false, true, g, s));
         if(cL > 65535) return HEFF_BAD_SHAPE;
         dim3 grid((unsigned)cdiv(cR, 128), (unsigned)cL);
-        env_mix_kernel<T, false><<<grid, 128, wsm, s>>>(X, Y, W, (int)d, (int)cR, (int)cL, (int)DL, (int)DR);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(env_mix_kernel<T, false>, grid, 128, wsm, s, X, Y, W, (int)d, (int)cR, (int)cL, (int)DL, (int)DR)));
         GemmArgs h{};
         h.M = (int)cL, h.N = (int)(cL * DL), h.K = (int)(d * cR), h.batch = 1;
         h.A = M2, h.lda = d * cR, h.B = Y, h.ldb = d * cR, h.C = out, h.ldc = cL;

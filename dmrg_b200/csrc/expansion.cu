@@ -27,6 +27,7 @@ __device__ __forceinline__ bool ex_nz(double2 w) { return w.x != 0.0 || w.y != 0
 
 template<class T>
 __global__ void expansion_mix_R(const T *__restrict__ X, const T *__restrict__ W, T *__restrict__ P, int S, int64_t cL, int64_t cR, int DL, int DR) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char ex_smem[];
     T        *sW = reinterpret_cast<T *>(ex_smem);
     const int nW = DL * DR * S * S;
@@ -104,8 +105,7 @@ int expansion_term(int side, typename Scalar<CPLX>::T *P, const typename Scalar<
     g.alpha = make_double2(alpha, 0.0);
     g.beta  = make_double2(0.0, 0.0);
     HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
-    expansion_mix_R<T><<<ex_grid(nP), 256, smem, s>>>(X, W, P, (int)S, cL, cR, (int)DL, (int)DR);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(expansion_mix_R<T>, ex_grid(nP), 256, smem, s, X, W, P, (int)S, cL, cR, (int)DL, (int)DR)));
     return HEFF_OK;
 }
 

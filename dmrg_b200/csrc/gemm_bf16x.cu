@@ -53,6 +53,7 @@ __device__ __forceinline__ void x_store(const XGemmArgs &p, int row, int n, floa
 //   warps 2-5:     epilogue of tile j from buffer (j & 1) while the MMAs of tile j+1 run in the other buffer
 __global__ void __launch_bounds__(X_THREADS, 1)
     gemm_bf16x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const XGemmArgs p) {
+    grid_wait();
     extern __shared__ __align__(1024) unsigned char xsm_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(xsm_raw) + 1023) & ~uintptr_t(1023));
     uint64_t      *full      = reinterpret_cast<uint64_t *>(smem + X_STAGES * X_STAGE_BYTES);
@@ -227,8 +228,7 @@ int gemm_bf16x(const CUtensorMap &tmA, const CUtensorMap &tmB, const XGemmArgs &
     const int64_t tiles = cdiv(a.M, X_BM) * cdiv(a.N, X_BN);
     if(tiles > 0x7fffffff) return HEFF_BAD_SHAPE;
     const int grid = (int)std::min<int64_t>(tiles, device_sm_count());  // persistent: one CTA per SM
-    gemm_bf16x_kernel<<<(unsigned)grid, X_THREADS, X_SMEM_BYTES, s>>>(tmA, tmB, a);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(gemm_bf16x_kernel, (unsigned)grid, X_THREADS, X_SMEM_BYTES, s, tmA, tmB, a)));
     return HEFF_OK;
 }
 

@@ -136,32 +136,15 @@ static int launch_gemm(const GemmArgs &a_in, const GemmPlan &pl, cudaStream_t st
     a.cluster = pl.cluster;
     a.units   = (int)units;
     gemm_fn_register(reinterpret_cast<const void *>(kern));
-    if(pl.cluster > 1) {
-        cudaLaunchConfig_t  lc = {};
-        cudaLaunchAttribute at[1];
-        at[0].id               = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)pl.cluster;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        lc.gridDim             = dim3((unsigned)units);
-        lc.blockDim            = dim3(G::THREADS);
-        lc.dynamicSmemBytes    = SM::BYTES;
-        lc.stream              = stream;
-        lc.attrs               = at;
-        lc.numAttrs            = 1;
-        HEFF_CUDA(cudaLaunchKernelEx(&lc, kern, (const GemmArgs)a));
-    } else {
-        const int64_t slots = (int64_t)device_sm_count() * per_sm;
-        kern<<<dim3((unsigned)(units < slots ? units : slots)), G::THREADS, SM::BYTES, stream>>>(a);
-        HEFF_LAUNCH_CHECK();
-    }
+    // a cluster launch has one CTA per unit; otherwise one persistent CTA per slot at most
+    const int64_t slots = pl.cluster > 1 ? units : (int64_t)device_sm_count() * per_sm;
+    HEFF_CUDA(launch_chained_cluster((unsigned)pl.cluster, kern, (unsigned)std::min(units, slots), G::THREADS, SM::BYTES, stream, a));
     count_launches(pl.split > 1 ? 2 : 1);
     if(pl.split > 1) {
         using SR = SplitReduce<CPLX, CFG>;
         const dim3 rgrid((unsigned)(tiles - pl.nfull), (unsigned)(SR::EPT / SR::EPB));
         gemm_fn_register(reinterpret_cast<const void *>(gemm_split_reduce_kernel<CPLX, CFG>));
-        gemm_split_reduce_kernel<CPLX, CFG><<<rgrid, G::THREADS, 0, stream>>>(a);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(gemm_split_reduce_kernel<CPLX, CFG>, rgrid, G::THREADS, 0, stream, a)));
     }
     return HEFF_OK;
 }

@@ -175,6 +175,7 @@ __device__ __forceinline__ GemmUnit gemm_unit(const GemmArgs &p, int u, int tile
 // cp.async (2 doubles or 1).
 template<bool CPLX, int CFG, bool TA, bool TB, int VEC>
 __global__ void __launch_bounds__(GemmTile<CPLX, CFG>::THREADS, GemmTile<CPLX, CFG>::MINB) gemm_f64_kernel(const GemmArgs p) {
+    grid_wait();
     using G  = GemmTile<CPLX, CFG>;
     using SM = GemmSmem<CPLX, CFG, TA, TB>;
     using T  = typename Scalar<CPLX>::T;
@@ -426,6 +427,7 @@ struct SplitReduce {
 };
 template<bool CPLX, int CFG>
 __global__ void __launch_bounds__(GemmTile<CPLX, CFG>::THREADS) gemm_split_reduce_kernel(const GemmArgs p) {
+    grid_wait();
     using G  = GemmTile<CPLX, CFG>;
     using T  = typename Scalar<CPLX>::T;
     using SR = SplitReduce<CPLX, CFG>;

@@ -45,6 +45,7 @@ __device__ __forceinline__ void z_set_scale(double mx, double extra, double *inv
 template<bool CPLX>
 __global__ void z_scale_k_kernel(const typename Scalar<CPLX>::T *__restrict__ src, int64_t rows, int64_t K, int64_t ld, double extra,
                                  double *__restrict__ inv, double *__restrict__ fac, int *bad) {
+    grid_wait();
     const int     lane = threadIdx.x & 31;
     const int64_t nw   = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for(int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
@@ -66,6 +67,7 @@ __global__ void z_scale_k_kernel(const typename Scalar<CPLX>::T *__restrict__ sr
 template<bool CPLX>
 __global__ void z_rowmax_m_kernel(const typename Scalar<CPLX>::T *__restrict__ src, int64_t rows, int64_t K, int64_t ld, int64_t kchunk,
                                   unsigned long long *rmax) {
+    grid_wait();
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if(r >= rows) return;
     const int64_t k0 = (int64_t)blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
@@ -78,6 +80,7 @@ __global__ void z_rowmax_m_kernel(const typename Scalar<CPLX>::T *__restrict__ s
     if(m > 0.0) atomicMax(rmax + r, (unsigned long long)__double_as_longlong(m));
 }
 __global__ void z_rowmax_fin_kernel(unsigned long long *rmax, int64_t rows, double extra, double *inv, double *fac, int *bad) {
+    grid_wait();
     for(int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
         const double m = __longlong_as_double((long long)rmax[r]);
         rmax[r]        = 0ull;  // ready for the next use
@@ -141,6 +144,7 @@ template<bool CPLX, bool BMODE>
 __global__ void __launch_bounds__(256) z_slice_k_kernel(const typename Scalar<CPLX>::T *__restrict__ src, int64_t rows, int64_t K, int64_t ld,
                                                          const double *__restrict__ inv, int8_t *__restrict__ planes, int64_t prow, int64_t kx, int ns,
                                                          int *bad) {
+    grid_wait();
     const int64_t ng = (K + 15) / 16, Kh = ng * 16, tot = rows * ng, plane = prow * kx;
     for(int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t g = e % ng, r = e / ng;
@@ -168,6 +172,7 @@ template<bool CPLX>
 __global__ void __launch_bounds__(ZM_THREADS) z_slice_m_kernel(const typename Scalar<CPLX>::T *__restrict__ src, int64_t rows, int64_t K,
                                                                 int64_t ld, const double *__restrict__ inv, int8_t *__restrict__ planes, int64_t kx,
                                                                 int ns, int *bad) {
+    grid_wait();
     using T = typename Scalar<CPLX>::T;
     __shared__ T  tile[ZM_TK][ZM_TR + 1];
     const int64_t ng = (K + 15) / 16, Kh = ng * 16, plane = rows * kx;
@@ -206,8 +211,7 @@ static int z_grid(int64_t n, int per_block = 256) {
 template<bool CPLX>
 int z_scale_kmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K, int64_t ld, double extra, ZPlanes &p, int *bad, cudaStream_t s) {
     if(rows <= 0) return HEFF_OK;
-    z_scale_k_kernel<CPLX><<<z_grid(rows * 32), 256, 0, s>>>(src, rows, K, ld, extra, p.inv, p.fac, bad);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(z_scale_k_kernel<CPLX>, z_grid(rows * 32), 256, 0, s, src, rows, K, ld, extra, p.inv, p.fac, bad)));
     return HEFF_OK;
 }
 
@@ -218,10 +222,8 @@ int z_scale_mmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
     const int64_t nchunks = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(K, 65535), (int64_t)device_sm_count() * 8 / rb));
     const int64_t kchunk  = cdiv(K, nchunks);
     if(rb > 0x7fffffff) return HEFF_BAD_SHAPE;
-    z_rowmax_m_kernel<CPLX><<<dim3((unsigned)rb, (unsigned)cdiv(K, kchunk)), 256, 0, s>>>(src, rows, K, ld, kchunk, p.rmax);
-    HEFF_LAUNCH_CHECK();
-    z_rowmax_fin_kernel<<<z_grid(rows), 256, 0, s>>>(p.rmax, rows, extra, p.inv, p.fac, bad);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(z_rowmax_m_kernel<CPLX>, dim3((unsigned)rb, (unsigned)cdiv(K, kchunk)), 256, 0, s, src, rows, K, ld, kchunk, p.rmax)));
+    HEFF_CUDA((launch_chained(z_rowmax_fin_kernel, z_grid(rows), 256, 0, s, p.rmax, rows, extra, p.inv, p.fac, bad)));
     return HEFF_OK;
 }
 
@@ -230,10 +232,9 @@ int z_slice_kmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
     if(rows <= 0) return HEFF_OK;
     const int64_t tot = rows * cdiv(K, 16);
     if(CPLX && bmode)
-        z_slice_k_kernel<CPLX, true><<<z_grid(tot), 256, 0, s>>>(src, rows, K, ld, p.inv, p.planes, p.rows, p.kx, p.nslice, bad);
+        HEFF_CUDA((launch_chained(z_slice_k_kernel<CPLX, true>, z_grid(tot), 256, 0, s, src, rows, K, ld, p.inv, p.planes, p.rows, p.kx, p.nslice, bad)));
     else
-        z_slice_k_kernel<CPLX, false><<<z_grid(tot), 256, 0, s>>>(src, rows, K, ld, p.inv, p.planes, p.rows, p.kx, p.nslice, bad);
-    HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(z_slice_k_kernel<CPLX, false>, z_grid(tot), 256, 0, s, src, rows, K, ld, p.inv, p.planes, p.rows, p.kx, p.nslice, bad)));
     return HEFF_OK;
 }
 
@@ -242,8 +243,7 @@ int z_slice_mmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
     if(rows <= 0) return HEFF_OK;
     const int64_t gx = cdiv(rows, ZM_TR), gy = cdiv(K, ZM_TK);
     if(gx > 0x7fffffff || gy > 65535) return HEFF_BAD_SHAPE;
-    z_slice_m_kernel<CPLX><<<dim3((unsigned)gx, (unsigned)gy), ZM_THREADS, 0, s>>>(src, rows, K, ld, p.inv, p.planes, p.kx, p.nslice, bad);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(z_slice_m_kernel<CPLX>, dim3((unsigned)gx, (unsigned)gy), ZM_THREADS, 0, s, src, rows, K, ld, p.inv, p.planes, p.kx, p.nslice, bad)));
     return HEFF_OK;
 }
 
@@ -409,6 +409,7 @@ __device__ __forceinline__ void z_epilogue_tsum(const ZGemmArgs &p, uint32_t tac
 template<int BN>
 __global__ void __launch_bounds__(Z_THREADS, 1)
     gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ZGemmArgs p) {
+    grid_wait();
     extern __shared__ __align__(1024) unsigned char zsm_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(zsm_raw) + 1023) & ~uintptr_t(1023));
     using Cfg                = ZCfg<BN>;
@@ -628,8 +629,7 @@ static int z_launch(const CUtensorMap &tA, const CUtensorMap &tB, const ZGemmArg
     const int64_t tiles = cdiv(a.M, Z_BM) * cdiv(a.N, BN);
     if(tiles > 0x7fffffff) return HEFF_BAD_SHAPE;
     const int grid = (int)std::min<int64_t>(tiles, device_sm_count());
-    gemm_i8_kernel<BN><<<(unsigned)grid, Z_THREADS, ZCfg<BN>::SMEM, s>>>(tA, tB, a);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(gemm_i8_kernel<BN>, (unsigned)grid, Z_THREADS, ZCfg<BN>::SMEM, s, tA, tB, a)));
     return HEFF_OK;
 }
 

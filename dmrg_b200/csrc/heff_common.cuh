@@ -29,6 +29,40 @@ void set_last_error_msg(const char *fmt, ...);
 // Launch check: picks up launch-configuration errors without synchronising.
 #define HEFF_LAUNCH_CHECK() HEFF_CUDA(cudaPeekAtLastError())
 
+// Chained launches (programmatic dependent launch).  A kernel launched with launch_chained may be set up on the device while
+// the kernel before it in the stream finishes; its first statement, grid_wait(), holds every thread until that kernel has
+// completed and its writes are visible.  Every thread of every chained kernel calls it before anything else, so a kernel
+// completes only after all that precede it, as without the attribute.  Measured on a chain of 1 us kernels: 4.1 us a kernel
+// with plain launches, 2.4 us chained; a GEMM of one k-tile 4.2 and 2.7 us.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template<class... P, class... A>
+cudaError_t launch_chained_cluster(unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    static_assert(sizeof...(P) == sizeof...(A), "one argument per parameter");
+    cudaLaunchConfig_t  lc = {};
+    cudaLaunchAttribute at[2];
+    lc.gridDim          = grid;
+    lc.blockDim         = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream           = stream;
+    at[0].id            = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs    = at;
+    lc.numAttrs = 1;
+    if(cluster > 1) {
+        at[1].id               = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = cluster;
+        at[1].val.clusterDim.y = 1;
+        at[1].val.clusterDim.z = 1;
+        lc.numAttrs            = 2;
+    }
+    return cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
+}
+template<class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    return launch_chained_cluster(1u, kernel, grid, block, smem, stream, args...);
+}
+
 template<bool CPLX>
 struct Scalar;
 template<>

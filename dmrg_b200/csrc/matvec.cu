@@ -34,6 +34,7 @@ int check_matvec_dims(const int64_t md[3], const int64_t wd[4], const int64_t ld
 // x'[a + cL*(s + S*b)] = x[s + S*(a + cL*b)]   (output-linear: coalesced writes)
 template<class T>
 __global__ void permute_mps_kernel(const T *__restrict__ x, T *__restrict__ xp, int64_t S, int64_t cL, int64_t n) {
+    grid_wait();
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = o % cL, r = o / cL, s = r % S, b = r / S;
         xp[o]           = x[s + S * (a + cL * b)];
@@ -43,6 +44,7 @@ __global__ void permute_mps_kernel(const T *__restrict__ x, T *__restrict__ xp, 
 // x'[o] for o in [o0, o1) (the x' columns (s,b) of a slab of b)
 template<class T>
 __global__ void permute_mps_range_kernel(const T *__restrict__ x, T *__restrict__ xp, int64_t S, int64_t cL, int64_t o0, int64_t o1) {
+    grid_wait();
     for(int64_t o = o0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < o1; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = o % cL, r = o / cL, s = r % S, b = r / S;
         xp[o]           = x[s + S * (a + cL * b)];
@@ -52,6 +54,7 @@ __global__ void permute_mps_range_kernel(const T *__restrict__ x, T *__restrict_
 // R'[b + cR*n + cR*DR*b'] = R[b + cR*(b' + cR*n)]
 template<class T>
 __global__ void permute_R_kernel(const T *__restrict__ R, T *__restrict__ Rp, int64_t cR, int64_t DR, int64_t n) {
+    grid_wait();
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = o % cR, r = o / cR, nn = r % DR, bp = r / DR;
         Rp[o]           = R[b + cR * (bp + cR * nn)];
@@ -74,6 +77,7 @@ constexpr int MIX_THREADS = 128;
 template<class T>
 __global__ void __launch_bounds__(MIX_THREADS) mix_kernel(const T *__restrict__ T1, T *__restrict__ T2, const T *__restrict__ W, int S, int cL,
                                                          int cR, int DL, int DR, int b0) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char mix_smem[];
     T        *sW  = reinterpret_cast<T *>(mix_smem);
     const int nW  = DL * DR * S * S;
@@ -125,8 +129,7 @@ static int grid_1d(int64_t n) {
 template<bool CPLX>
 int permute_R(const typename Scalar<CPLX>::T *R, typename Scalar<CPLX>::T *Rp, const MatvecDims &d, cudaStream_t s) {
     const int64_t n = d.size_Rp();
-    permute_R_kernel<<<grid_1d(n), 256, 0, s>>>(R, Rp, d.cR, d.DR, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(permute_R_kernel<typename Scalar<CPLX>::T>, grid_1d(n), 256, 0, s, R, Rp, d.cR, d.DR, n)));
     return HEFF_OK;
 }
 
@@ -148,8 +151,7 @@ static int launch_mix(const MatvecDims &d, const typename Scalar<CPLX>::T *T1, t
     if(nb > 65535) return HEFF_BAD_SHAPE;
     if(nb == 0) return HEFF_OK;
     dim3 grid((unsigned)cdiv(d.cL, MIX_THREADS), (unsigned)nb);
-    mix_kernel<T><<<grid, MIX_THREADS, smem, s>>>(T1, T2, W, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL, (int)d.DR, (int)b0);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(mix_kernel<T>, grid, MIX_THREADS, smem, s, T1, T2, W, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL, (int)d.DR, (int)b0)));
     return HEFF_OK;
 }
 
@@ -159,8 +161,7 @@ int matvec_fp64(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename
                 cudaEvent_t *ev) {
     const int64_t n = d.size_mps();
     if(ev) HEFF_CUDA(cudaEventRecord(ev[0], s));
-    permute_mps_kernel<<<grid_1d(n), 256, 0, s>>>(x, ws.xp, d.S, d.cL, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(permute_mps_kernel<typename Scalar<CPLX>::T>, grid_1d(n), 256, 0, s, x, ws.xp, d.S, d.cL, n)));
     count_launches(2);  // the permutation and the MPO mix below (the GEMM launcher counts its own kernels)
     if(ev) HEFF_CUDA(cudaEventRecord(ev[1], s));
     GemmArgs g1{};
@@ -209,8 +210,7 @@ template<bool CPLX>
 int matvec_left_stages(const MatvecDims &d, const typename Scalar<CPLX>::T *x, const typename Scalar<CPLX>::T *L, const typename Scalar<CPLX>::T *W,
                        typename Scalar<CPLX>::T *out, typename Scalar<CPLX>::T *xp, typename Scalar<CPLX>::T *T1, double alpha, cudaStream_t s) {
     const int64_t n = d.size_mps();
-    permute_mps_kernel<<<grid_1d(n), 256, 0, s>>>(x, xp, d.S, d.cL, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(permute_mps_kernel<typename Scalar<CPLX>::T>, grid_1d(n), 256, 0, s, x, xp, d.S, d.cL, n)));
     GemmArgs g1{};
     g1.M     = (int)(d.cL * d.DL);
     g1.N     = (int)(d.S * d.cR);
@@ -259,8 +259,7 @@ int matvec_fp64_host(const MatvecDims &d, const typename Scalar<CPLX>::T *xh, ty
         cudaStream_t s = cs[c & 1];
         HEFF_CUDA(cudaStreamWaitEvent(s, hp.ev[1 + c], 0));
         const int64_t o0 = d.cL * d.S * b0, o1 = d.cL * d.S * b1;
-        permute_mps_range_kernel<<<grid_1d(o1 - o0), 256, 0, s>>>(dx, ws.xp, d.S, d.cL, o0, o1);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(permute_mps_range_kernel<T>, grid_1d(o1 - o0), 256, 0, s, dx, ws.xp, d.S, d.cL, o0, o1)));
         GemmArgs g1{};
         g1.M = (int)(d.cL * d.DL), g1.N = (int)(d.S * (b1 - b0)), g1.K = (int)d.cL, g1.batch = 1;
         g1.A = L, g1.lda = d.cL, g1.B = ws.xp + o0, g1.ldb = d.cL, g1.C = ws.T1 + d.cL * d.DL * d.S * b0, g1.ldc = d.cL * d.DL;
@@ -299,6 +298,7 @@ constexpr int DOT_BLOCKS = 1024;
 template<bool CPLX>
 __global__ void dot_partial_kernel(const typename Scalar<CPLX>::T *__restrict__ x, const typename Scalar<CPLX>::T *__restrict__ y, int64_t n,
                                    double *partials) {
+    grid_wait();
     __shared__ double sre[256], sim[256];
     double            re = 0, im = 0;
     for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -327,6 +327,7 @@ __global__ void dot_partial_kernel(const typename Scalar<CPLX>::T *__restrict__ 
 }
 template<bool CPLX>
 __global__ void dot_final_kernel(const double *partials, int nb, typename Scalar<CPLX>::T *out) {
+    grid_wait();
     __shared__ double sre[256], sim[256];
     double            re = 0, im = 0;
     for(int i = threadIdx.x; i < nb; i += 256) {
@@ -355,10 +356,8 @@ template<bool CPLX>
 int dot_device(const typename Scalar<CPLX>::T *x, const typename Scalar<CPLX>::T *y, int64_t n, typename Scalar<CPLX>::T *out, double *partials,
                cudaStream_t s) {
     int nb = (int)std::min<int64_t>(DOT_BLOCKS, std::max<int64_t>(1, (n + 255) / 256));
-    dot_partial_kernel<CPLX><<<nb, 256, 0, s>>>(x, y, n, partials);
-    HEFF_LAUNCH_CHECK();
-    dot_final_kernel<CPLX><<<1, 256, 0, s>>>(partials, nb, out);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(dot_partial_kernel<CPLX>, nb, 256, 0, s, x, y, n, partials)));
+    HEFF_CUDA((launch_chained(dot_final_kernel<CPLX>, 1, 256, 0, s, partials, nb, out)));
     return HEFF_OK;
 }
 
@@ -369,8 +368,7 @@ const void *permute_kernel_fn(bool cplx) {
 template<bool CPLX>
 int permute_mps(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename Scalar<CPLX>::T *xp, cudaStream_t s) {
     const int64_t n = d.size_mps();
-    permute_mps_kernel<<<grid_1d(n), 256, 0, s>>>(x, xp, d.S, d.cL, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(permute_mps_kernel<typename Scalar<CPLX>::T>, grid_1d(n), 256, 0, s, x, xp, d.S, d.cL, n)));
     return HEFF_OK;
 }
 template<bool CPLX>

@@ -115,6 +115,7 @@ __device__ __forceinline__ double im_of(double2 v) { return v.y; }
 template<bool CPLX>
 __global__ void split_L_kernel(const typename Scalar<CPLX>::T *__restrict__ L, __nv_bfloat16 *__restrict__ A1, int64_t cL, int64_t M1, int64_t Kp1,
                                int64_t Kx1) {
+    grid_wait();
     const int64_t tot = cL * M1;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = e % cL, r = e / cL;
@@ -126,6 +127,7 @@ __global__ void split_L_kernel(const typename Scalar<CPLX>::T *__restrict__ L, _
 template<bool CPLX>
 __global__ void split_R_kernel(const typename Scalar<CPLX>::T *__restrict__ Rp, __nv_bfloat16 *__restrict__ B2, int64_t K2, int64_t cR, int64_t Kp2,
                                int64_t Kx2) {
+    grid_wait();
     const int64_t tot = K2 * cR;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t k = e % K2, bp = e / K2;
@@ -139,6 +141,7 @@ __global__ void split_R_kernel(const typename Scalar<CPLX>::T *__restrict__ Rp, 
 template<bool CPLX>
 __global__ void __launch_bounds__(256) split_x_kernel(const typename Scalar<CPLX>::T *__restrict__ x, __nv_bfloat16 *__restrict__ B1, int64_t S,
                                                       int64_t cL, int64_t N1, int64_t Kp1, int64_t Kx1, int ta) {
+    grid_wait();
     using T = typename Scalar<CPLX>::T;
     extern __shared__ __align__(16) unsigned char sx_smem[];
     T            *sx  = reinterpret_cast<T *>(sx_smem);  // [S][ta]
@@ -189,6 +192,7 @@ template<bool CPLX, int TA>
 __global__ void __launch_bounds__(32 * TA) mix_mixed_kernel(const float *__restrict__ T1, const unsigned char *__restrict__ wl, int wl_bytes,
                                                            __nv_bfloat16 *__restrict__ A2, int S, int cL, int cR, int DL, int DR, int64_t M1,
                                                            int64_t N1, int64_t Kp2, int64_t Kx2) {
+    grid_wait();
     using T                 = typename Scalar<CPLX>::T;
     constexpr int SSTR      = mx_sstr<TA>();
     constexpr int NTHREADS  = 32 * TA;
@@ -436,18 +440,15 @@ static int mixed_setup(heff_op *op) {
     // cleared whenever the layout is (re)built, since the pool may hold another shape's values
     HEFF_CUDA(cudaMemsetAsync(m->pool, 0, z.b[0] + z.b[1] + z.b[2] + z.b[3], s));
     HEFF_CUDA(cudaMemsetAsync(m->err, 0, sizeof(int), s));
-    split_L_kernel<CPLX><<<g1(m->K1 * m->M1), 256, 0, s>>>(reinterpret_cast<const T *>(op->L), m->A1, d.cL, m->M1, m->Kp1, m->Kx1);
-    HEFF_LAUNCH_CHECK();
-    split_R_kernel<CPLX><<<g1(m->K2 * m->N2), 256, 0, s>>>(reinterpret_cast<const T *>(op->Rp), m->B2, m->K2, d.cR, m->Kp2, m->Kx2);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(split_L_kernel<CPLX>, g1(m->K1 * m->M1), 256, 0, s, reinterpret_cast<const T *>(op->L), m->A1, d.cL, m->M1, m->Kp1, m->Kx1)));
+    HEFF_CUDA((launch_chained(split_R_kernel<CPLX>, g1(m->K2 * m->N2), 256, 0, s, reinterpret_cast<const T *>(op->Rp), m->B2, m->K2, d.cR, m->Kp2, m->Kx2)));
     HEFF_TRY(make_tmap_bf16(&m->tA1, m->A1, m->M1, m->Kx1, m->Kx1, X_BM));
     HEFF_TRY(make_tmap_bf16(&m->tB1, m->B1, cf * m->N1, m->Kx1, m->Kx1, X_BN));
     HEFF_TRY(make_tmap_bf16(&m->tA2, m->A2, m->M2, m->Kx2, m->Kx2, X_BM));
     HEFF_TRY(make_tmap_bf16(&m->tB2, m->B2, cf * m->N2, m->Kx2, m->Kx2, X_BN));
 
     m->wl_bytes = (int)wlist_bytes((int)d.DL, (int)d.DR, (int)d.S, sizeof(T));
-    wlist_global_kernel<T><<<1, 32, 0, s>>>(reinterpret_cast<const T *>(op->W), (int)d.DL, (int)d.DR, (int)d.S, m->wl);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(wlist_global_kernel<T>, 1, 32, 0, s, reinterpret_cast<const T *>(op->W), (int)d.DL, (int)d.DR, (int)d.S, m->wl)));
     const int    ta       = mx_ta(d.DL * d.S, cf);
     const size_t mix_smem = mx_smem(d.DL * d.S, cf, ta, m->wl_bytes);
     if(mix_smem > 200 * 1024) return HEFF_BAD_SHAPE;
@@ -468,9 +469,7 @@ static int mixed_apply_impl(heff_op *op, const void *x, void *y) {
     // slab width: 256 values of a, fewer for large merged spins so the tile stays within 48 KB
     const int ta = (int)std::max<int64_t>(32, std::min<int64_t>(256, (int64_t)(48 * 1024 / (sizeof(T) * d.S)) / 32 * 32));
     if(d.cR > 65535 || (size_t)d.S * ta * sizeof(T) > 48 * 1024) return HEFF_BAD_SHAPE;
-    split_x_kernel<CPLX><<<dim3((unsigned)cdiv(d.cL, ta), (unsigned)d.cR), 256, (size_t)d.S * ta * sizeof(T), s>>>(
-        reinterpret_cast<const T *>(x), m->B1, d.S, d.cL, m->N1, m->Kp1, m->Kx1, ta);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(split_x_kernel<CPLX>, dim3((unsigned)cdiv(d.cL, ta), (unsigned)d.cR), 256, (size_t)d.S * ta * sizeof(T), s,  reinterpret_cast<const T *>(x), m->B1, d.S, d.cL, m->N1, m->Kp1, m->Kx1, ta)));
     XGemmArgs g1a{};
     g1a.M = (int)m->M1, g1a.N = (int)(cf * m->N1), g1a.K = (int)m->Kx1, g1a.C = m->T1, g1a.ldc = m->M1, g1a.mode = X_OUT_F32, g1a.err = m->err;
     HEFF_TRY(gemm_bf16x(m->tA1, m->tB1, g1a, s));
@@ -479,12 +478,9 @@ static int mixed_apply_impl(heff_op *op, const void *x, void *y) {
     if(d.cR / MX_TB + 1 > 65535) return HEFF_BAD_SHAPE;
     dim3 grid((unsigned)cdiv(d.cL, mta), (unsigned)cdiv(d.cR, MX_TB));
     if(mta == 16)
-        mix_mixed_kernel<CPLX, 16><<<grid, 32 * 16, mix_smem, s>>>(m->T1, m->wl, m->wl_bytes, m->A2, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL,
-                                                                  (int)d.DR, m->M1, m->N1, m->Kp2, m->Kx2);
+        HEFF_CUDA((launch_chained(mix_mixed_kernel<CPLX, 16>, grid, 32 * 16, mix_smem, s, m->T1, m->wl, m->wl_bytes, m->A2, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL, (int)d.DR, m->M1, m->N1, m->Kp2, m->Kx2)));
     else
-        mix_mixed_kernel<CPLX, 8><<<grid, 32 * 8, mix_smem, s>>>(m->T1, m->wl, m->wl_bytes, m->A2, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL,
-                                                                (int)d.DR, m->M1, m->N1, m->Kp2, m->Kx2);
-    HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(mix_mixed_kernel<CPLX, 8>, grid, 32 * 8, mix_smem, s, m->T1, m->wl, m->wl_bytes, m->A2, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL, (int)d.DR, m->M1, m->N1, m->Kp2, m->Kx2)));
     XGemmArgs g2{};
     g2.M = (int)m->M2, g2.N = (int)(cf * m->N2), g2.K = (int)m->Kx2, g2.C = y, g2.ldc = m->M2, g2.err = m->err;
     g2.mode   = CPLX ? X_OUT_C128 : X_OUT_F64;

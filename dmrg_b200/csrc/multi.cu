@@ -35,6 +35,7 @@ __device__ __forceinline__ bool sm_nz(double2 w) { return w.x != 0.0 || w.y != 0
 template<class T, bool LAST>
 __global__ void site_mix_kernel(const T *__restrict__ in, T *__restrict__ out, const T *__restrict__ W, int Din, int Dout, int d, int64_t cL,
                                 int64_t cR, int64_t S, int64_t P) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char sm_smem[];
     T        *sW = reinterpret_cast<T *>(sm_smem);
     const int nW = Din * Dout * d * d;
@@ -70,6 +71,7 @@ static int mm_grid(int64_t n) {
 
 template<class T>
 __global__ void mm_permute_kernel(const T *__restrict__ x, T *__restrict__ xp, int64_t S, int64_t cL, int64_t n) {
+    grid_wait();
     // xp[a + cL (s + S b)] = x[s + S (a + cL b)]
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = o % cL, r = o / cL, s = r % S, b = r / S;
@@ -110,8 +112,7 @@ int matvec_multi(const MultiDims &md, const typename Scalar<CPLX>::T *x, typenam
     T            *xp    = scratch;
     T            *buf[2] = {xp + pad(n), xp + pad(n) + pad(n * md.Dmax)};
     const int64_t D0 = md.dims[0], DK = md.dims[4 * (md.nmpo - 1) + 1];
-    mm_permute_kernel<T><<<mm_grid(n), 256, 0, s>>>(x, xp, S, cL, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(mm_permute_kernel<T>, mm_grid(n), 256, 0, s, x, xp, S, cL, n)));
     GemmArgs g1{};
     g1.M = (int)(cL * D0), g1.N = (int)(S * cR), g1.K = (int)cL, g1.batch = 1;
     g1.A = L, g1.lda = cL, g1.B = xp, g1.ldb = cL, g1.C = buf[0], g1.ldc = cL * D0;
@@ -126,10 +127,9 @@ int matvec_multi(const MultiDims &md, const typename Scalar<CPLX>::T *x, typenam
         if(smem > 48 * 1024) return HEFF_BAD_SHAPE;
         const int64_t npts = cL * cR * S / w[2];
         if(last)
-            site_mix_kernel<T, true><<<mm_grid(npts), 256, smem, s>>>(buf[cur], buf[cur ^ 1], W[i], (int)w[0], (int)w[1], (int)w[2], cL, cR, S, P);
+            HEFF_CUDA((launch_chained(site_mix_kernel<T, true>, mm_grid(npts), 256, smem, s, buf[cur], buf[cur ^ 1], W[i], (int)w[0], (int)w[1], (int)w[2], cL, cR, S, P)));
         else
-            site_mix_kernel<T, false><<<mm_grid(npts), 256, smem, s>>>(buf[cur], buf[cur ^ 1], W[i], (int)w[0], (int)w[1], (int)w[2], cL, cR, S, P);
-        HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(site_mix_kernel<T, false>, mm_grid(npts), 256, smem, s, buf[cur], buf[cur ^ 1], W[i], (int)w[0], (int)w[1], (int)w[2], cL, cR, S, P)));
         cur ^= 1;
         P *= w[2];
     }

@@ -37,6 +37,7 @@ __device__ __forceinline__ double2 pc_scale(double2 a, double f) { return make_d
 template<class T>
 __global__ void diag_kernel(const T *__restrict__ L, const T *__restrict__ Rp, const T *__restrict__ W, int64_t S, int64_t cL, int64_t cR, int DL,
                             int DR, T *__restrict__ out) {
+    grid_wait();
     const int64_t n = S * cL * cR;
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = o % S, a = (o / S) % cL, b = o / (S * cL);
@@ -54,6 +55,7 @@ __global__ void diag_kernel(const T *__restrict__ L, const T *__restrict__ Rp, c
 
 template<class T>
 __global__ void multpc_kernel(const T *__restrict__ x, const T *__restrict__ diag, double shift, T *__restrict__ y, int64_t n) {
+    grid_wait();
     const double floor_ = 1e-10 * fmax(fabs(shift), 1.0);
     for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double den = pc_re(diag[i]) - shift;
@@ -89,6 +91,7 @@ __device__ __forceinline__ double2 pc_from_real<double2>(double v) { return make
 template<class T>
 __global__ void jcb_extract_kernel(const T *__restrict__ L, const T *__restrict__ Rp, const T *__restrict__ W, int64_t S, int64_t cL, int64_t cR,
                                    int DL, int DR, int64_t bs, int64_t nb, double shift, T *__restrict__ blocks) {
+    grid_wait();
     const int64_t n = S * cL * cR, per = bs * bs, tot = nb * per;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t k = e / per, rem = e - k * per, i = rem % bs, j = rem / bs;
@@ -120,6 +123,7 @@ __host__ __device__ constexpr size_t jcb_r16(size_t b) { return (b + 15) / 16 * 
 // as column interchanges in reverse order.
 template<class T, bool SMEM>
 __global__ void __launch_bounds__(256) jcb_invert_kernel(T *__restrict__ blocks, int bs, int *__restrict__ singular) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char jcb_smem[];
     // carve (every piece 16-byte aligned; jcb_smem_fixed gives the same total)
     const size_t o_perm = jcb_r16(sizeof(T) * bs), o_rv = o_perm + jcb_r16(sizeof(int) * bs), o_ri = o_rv + 64, o_sinv = o_ri + 32,
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(256) jcb_invert_kernel(T *__restrict__ blocks,
 // coalesced along rows).
 template<class T>
 __global__ void __launch_bounds__(256) jcb_apply_kernel(const T *__restrict__ inv, const T *__restrict__ x, T *__restrict__ y, int bs, int64_t n) {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char jcb_smem[];
     T            *xs  = reinterpret_cast<T *>(jcb_smem);
     const int64_t off = (int64_t)blockIdx.x * bs;
@@ -277,18 +282,15 @@ static int jcb_build(heff_op *op, double shift) {
     HEFF_CUDA(cudaMemsetAsync(sing, 0, sizeof(int), op->stream));
     const int64_t tot = nb * bs * bs;
     const int64_t g   = std::min<int64_t>((tot + 255) / 256, (int64_t)device_sm_count() * 16);
-    jcb_extract_kernel<T><<<(int)std::max<int64_t>(g, 1), 256, 0, op->stream>>>(reinterpret_cast<const T *>(op->L), reinterpret_cast<const T *>(op->Rp),
-                                                                               reinterpret_cast<const T *>(op->W), d.S, d.cL, d.cR, (int)d.DL, (int)d.DR,
-                                                                               bs, nb, shift, blocks);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(jcb_extract_kernel<T>, (int)std::max<int64_t>(g, 1), 256, 0, op->stream, reinterpret_cast<const T *>(op->L), reinterpret_cast<const T *>(op->Rp), reinterpret_cast<const T *>(op->W), d.S, d.cL, d.cR, (int)d.DL, (int)d.DR, bs, nb, shift, blocks)));
     const size_t fixed = jcb_smem_fixed((int)bs, es);
     const size_t full  = fixed + (size_t)bs * bs * es;
     if(nb > 0x7fffffffLL) return HEFF_BAD_SHAPE;
     if(full <= 200 * 1024) {
         HEFF_CUDA(cudaFuncSetAttribute(jcb_invert_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)full));
-        jcb_invert_kernel<T, true><<<(unsigned)nb, 256, full, op->stream>>>(blocks, (int)bs, sing);
+        HEFF_CUDA((launch_chained(jcb_invert_kernel<T, true>, (unsigned)nb, 256, full, op->stream, blocks, (int)bs, sing)));
     } else {
-        jcb_invert_kernel<T, false><<<(unsigned)nb, 256, fixed, op->stream>>>(blocks, (int)bs, sing);
+        HEFF_CUDA((launch_chained(jcb_invert_kernel<T, false>, (unsigned)nb, 256, fixed, op->stream, blocks, (int)bs, sing)));
     }
     HEFF_LAUNCH_CHECK();
     op->jcb_ready = true;
@@ -300,9 +302,7 @@ template<class T>
 static int jcb_apply(heff_op *op, const void *x, void *y) {
     const int64_t n = op->d.size_mps(), bs = op->jcb_block, nb = (n + bs - 1) / bs;
     const T      *blocks = reinterpret_cast<const T *>(reinterpret_cast<const unsigned char *>(op->jcb) + 256);
-    jcb_apply_kernel<T><<<(unsigned)nb, 256, (size_t)bs * sizeof(T), op->stream>>>(blocks, reinterpret_cast<const T *>(x), reinterpret_cast<T *>(y),
-                                                                                   (int)bs, n);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(jcb_apply_kernel<T>, (unsigned)nb, 256, (size_t)bs * sizeof(T), op->stream, blocks, reinterpret_cast<const T *>(x), reinterpret_cast<T *>(y), (int)bs, n)));
     return HEFF_OK;
 }
 
@@ -330,14 +330,9 @@ int op_diagonal_ready(heff_op *op) {
         op->diag_cap = n;
     }
     if(op->cplx)
-        diag_kernel<double2><<<pc_grid(n), 256, 0, op->stream>>>(reinterpret_cast<const double2 *>(op->L), reinterpret_cast<const double2 *>(op->Rp),
-                                                                  reinterpret_cast<const double2 *>(op->W), d.S, d.cL, d.cR, (int)d.DL, (int)d.DR,
-                                                                  reinterpret_cast<double2 *>(op->diag));
+        HEFF_CUDA((launch_chained(diag_kernel<double2>, pc_grid(n), 256, 0, op->stream, reinterpret_cast<const double2 *>(op->L), reinterpret_cast<const double2 *>(op->Rp), reinterpret_cast<const double2 *>(op->W), d.S, d.cL, d.cR, (int)d.DL, (int)d.DR, reinterpret_cast<double2 *>(op->diag))));
     else
-        diag_kernel<double><<<pc_grid(n), 256, 0, op->stream>>>(reinterpret_cast<const double *>(op->L), reinterpret_cast<const double *>(op->Rp),
-                                                                 reinterpret_cast<const double *>(op->W), d.S, d.cL, d.cR, (int)d.DL, (int)d.DR,
-                                                                 reinterpret_cast<double *>(op->diag));
-    HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(diag_kernel<double>, pc_grid(n), 256, 0, op->stream, reinterpret_cast<const double *>(op->L), reinterpret_cast<const double *>(op->Rp), reinterpret_cast<const double *>(op->W), d.S, d.cL, d.cR, (int)d.DL, (int)d.DR, reinterpret_cast<double *>(op->diag))));
     op->diag_ready = true;
     return HEFF_OK;
 }
@@ -354,12 +349,9 @@ int op_multpc(heff_op *op, const void *x, void *y, double shift) {
     HEFF_TRY(op_diagonal_ready(op));
     const int64_t n = op->d.size_mps();
     if(op->cplx)
-        multpc_kernel<double2><<<pc_grid(n), 256, 0, op->stream>>>(reinterpret_cast<const double2 *>(x), reinterpret_cast<const double2 *>(op->diag),
-                                                                    shift, reinterpret_cast<double2 *>(y), n);
+        HEFF_CUDA((launch_chained(multpc_kernel<double2>, pc_grid(n), 256, 0, op->stream, reinterpret_cast<const double2 *>(x), reinterpret_cast<const double2 *>(op->diag), shift, reinterpret_cast<double2 *>(y), n)));
     else
-        multpc_kernel<double><<<pc_grid(n), 256, 0, op->stream>>>(reinterpret_cast<const double *>(x), reinterpret_cast<const double *>(op->diag), shift,
-                                                                   reinterpret_cast<double *>(y), n);
-    HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(multpc_kernel<double>, pc_grid(n), 256, 0, op->stream, reinterpret_cast<const double *>(x), reinterpret_cast<const double *>(op->diag), shift, reinterpret_cast<double *>(y), n)));
     return HEFF_OK;
 }
 

@@ -442,6 +442,7 @@ template<class T>
 __global__ void __launch_bounds__(JTHR) jacobi_round_kernel(T *__restrict__ G, int64_t ldg, int m, T *__restrict__ V, int64_t ldv, int nv, int B,
                                                            int round, double tol, double floor_abs, const int *__restrict__ colmap,
                                                            double *__restrict__ gmax_out, int *__restrict__ rotated, int CL) {
+    grid_wait();
     using S  = JS<T>;
     using JK = JPairBlock<T>;
     constexpr int RC = S::ROWS;
@@ -559,6 +560,7 @@ constexpr size_t jacobi_whole_bytes() {
 template<class T, int P>
 __global__ void __launch_bounds__(jw_thr(P), 1) jacobi_whole_kernel(const T *A, int64_t lda, int adjoint, T *X, int64_t ldx, int m, int n, T *V, double tol,
                                                                    int max_sweeps, double *__restrict__ sig, int *__restrict__ sweeps_out) {
+    grid_wait();
     using S  = JS<T>;
     using JK = JWholeBlock<T, P>;
     constexpr int THR = jw_thr(P);
@@ -664,6 +666,7 @@ __global__ void __launch_bounds__(jw_thr(P), 1) jacobi_whole_kernel(const T *A, 
 // sigma_j = ||G_j||_2 (column norms), one warp per column.
 template<class T>
 __global__ void col_norms_kernel(const T *__restrict__ G, int64_t ldg, int m, int n, double *__restrict__ sig) {
+    grid_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
     if(w >= n) return;
     double acc = 0;
@@ -674,6 +677,7 @@ __global__ void col_norms_kernel(const T *__restrict__ G, int64_t ldg, int m, in
 
 // Stable descending order of the column norms: ord[rank of column i] = i (a NaN sorts last).
 __global__ void col_order_kernel(const double *__restrict__ sig, int n, int *__restrict__ ord) {
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     const double a = sig[i] >= 0 ? sig[i] : -1.0;
@@ -690,6 +694,7 @@ __global__ void col_order_kernel(const double *__restrict__ sig, int n, int *__r
 template<class T>
 __global__ void copy_pad_kernel(const T *__restrict__ A, int64_t lda, int rows, int cols, T *__restrict__ G, int64_t ldg, int npad,
                                 const int *__restrict__ ord) {
+    grid_wait();
     const int64_t tot = (int64_t)ldg * npad;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = e % ldg, c = e / ldg;
@@ -701,6 +706,7 @@ __global__ void copy_pad_kernel(const T *__restrict__ A, int64_t lda, int rows, 
 template<class T, bool UPPER>
 __global__ void __launch_bounds__(256) adjoint_kernel(const T *__restrict__ X, int64_t ldx, int xrows, int xcols, T *__restrict__ Y, int64_t ldy, int yrows,
                                                      int ycols) {
+    grid_wait();
     __shared__ T tile[32][33];
     const int    x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5;  // Y rows from y0, columns from x0
     for(int c = w; c < 32; c += 8) {
@@ -714,6 +720,7 @@ __global__ void __launch_bounds__(256) adjoint_kernel(const T *__restrict__ X, i
 
 template<class T>
 __global__ void eye_kernel(T *__restrict__ V, int64_t ldv, int npad) {
+    grid_wait();
     const int64_t tot = (int64_t)ldv * npad;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x)
         V[e] = (e % ldv == e / ldv) ? JS<T>::one() : JS<T>::zero();
@@ -725,6 +732,7 @@ template<class T, bool LADJ, bool RADJ>
 __global__ void take_columns_kernel(const T *__restrict__ W, int64_t ldw, int rows, const T *__restrict__ V, int64_t ldv, int n, const int *__restrict__ perm,
                                     const double *__restrict__ sig, int k, double *__restrict__ Sout, T *__restrict__ left, int64_t ldl, int lrows,
                                     T *__restrict__ right, int64_t ldr) {
+    grid_wait();
     const int64_t tl = (int64_t)lrows * k, tot = tl + (int64_t)n * k;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const bool    lt = e < tl;
@@ -751,6 +759,7 @@ __global__ void take_columns_kernel(const T *__restrict__ W, int64_t ldw, int ro
 // B (k x n, leading dim k)[i, ord[c]] = conj(X[c, i]);  ord may be nullptr (identity)
 template<class T>
 __global__ void adjoint_rows_kernel(const T *__restrict__ X, int64_t ldx, int n, int k, const int *__restrict__ ord, T *__restrict__ B) {
+    grid_wait();
     const int64_t tot = (int64_t)n * k;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t c = e / k, i = e % k;
@@ -760,6 +769,7 @@ __global__ void adjoint_rows_kernel(const T *__restrict__ X, int64_t ldx, int n,
 // out[ord[c], i] = X[c, i]
 template<class T>
 __global__ void scatter_rows_kernel(const T *__restrict__ X, int64_t ldx, int n, int k, const int *__restrict__ ord, T *__restrict__ out, int64_t ldo) {
+    grid_wait();
     const int64_t tot = (int64_t)n * k;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = e / n, c = e % n;
@@ -819,6 +829,7 @@ struct QrPanel {
 };
 template<class T>
 __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T *__restrict__ G, int64_t ldg, int M, int j0, int w, T *__restrict__ Tout, int CL) {
+    grid_wait();
     using S           = JS<T>;
     constexpr int RPT = QrPanel<T>::RPT;
     __shared__ T      s_red[QrPanel<T>::THR_MAX / 32][QW];
@@ -985,6 +996,7 @@ __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T
 template<class T, bool ADJ>
 __global__ void __launch_bounds__(256) qr_apply_kernel(const T *__restrict__ G, int64_t ldg, int M, int j0, const T *__restrict__ Tm, T *__restrict__ A,
                                                       int64_t lda, int nc) {
+    grid_wait();
     using S = JS<T>;
     constexpr bool C = !std::is_same<T, double>::value;
     __shared__ T     sW[8][QW][QW + 1], sX[QW][QW + 1], sT[QW][QW + 1];
@@ -1125,27 +1137,10 @@ static int qr_factor(T *G, int64_t ldg, int M, int N, T *Tf, cudaStream_t s) {
         int       CL  = 1;
         while(CL * RPT * thr < rows) CL *= 2;
         T *Tp = Tf + (int64_t)(j0 / QW) * QW * QW;
-        if(CL == 1) {
-            qr_panel_kernel<T><<<1, thr + 32, 0, s>>>(G, ldg, M, j0, w, Tp, 1);
-            HEFF_LAUNCH_CHECK();
-        } else {
-            cudaLaunchConfig_t  lc = {};
-            cudaLaunchAttribute at[1];
-            at[0].id               = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)CL;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            lc.gridDim             = dim3((unsigned)CL);
-            lc.blockDim            = dim3((unsigned)(thr + 32));
-            lc.stream              = s;
-            lc.attrs               = at;
-            lc.numAttrs            = 1;
-            HEFF_CUDA(cudaLaunchKernelEx(&lc, qr_panel_kernel<T>, G, ldg, M, j0, w, Tp, CL));
-        }
+        HEFF_CUDA((launch_chained_cluster((unsigned)CL, qr_panel_kernel<T>, CL, thr + 32, 0, s, G, ldg, M, j0, w, Tp, CL)));
         const int rest = N - j0 - w;
         if(rest > 0) {
-            qr_apply_kernel<T, true><<<(rest + QW - 1) / QW, 256, 0, s>>>(G, ldg, M, j0, Tp, G + ldg * (int64_t)(j0 + w), ldg, rest);
-            HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(qr_apply_kernel<T, true>, (rest + QW - 1) / QW, 256, 0, s, G, ldg, M, j0, Tp, G + ldg * (int64_t)(j0 + w), ldg, rest)));
         }
     }
     return HEFF_OK;
@@ -1154,8 +1149,7 @@ static int qr_factor(T *G, int64_t ldg, int M, int N, T *Tf, cudaStream_t s) {
 template<class T>
 static int qr_apply_q(const T *G, int64_t ldg, int M, int N, const T *Tf, T *A, int64_t lda, int nc, cudaStream_t s) {
     for(int j0 = (N - 1) / QW * QW; j0 >= 0; j0 -= QW) {
-        qr_apply_kernel<T, false><<<(nc + QW - 1) / QW, 256, 0, s>>>(G, ldg, M, j0, Tf + (int64_t)(j0 / QW) * QW * QW, A, lda, nc);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(qr_apply_kernel<T, false>, (nc + QW - 1) / QW, 256, 0, s, G, ldg, M, j0, Tf + (int64_t)(j0 / QW) * QW * QW, A, lda, nc)));
     }
     return HEFF_OK;
 }
@@ -1201,10 +1195,8 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     int          *cmap = perm + npad;  // column order of the current sweep (block b = columns cmap[16 b .. 16 b + 15])
     int          *cord = cmap + npad;  // order of A's columns in G
     auto norms_order = [&](const T *W, int64_t ldw, int rows, int cols, double *nrm, int *ord) -> int {
-        col_norms_kernel<T><<<(cols * 32 + 255) / 256, 256, 0, s>>>(W, ldw, rows, cols, nrm);
-        HEFF_LAUNCH_CHECK();
-        col_order_kernel<<<(cols + 127) / 128, 128, 0, s>>>(nrm, cols, ord);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(col_norms_kernel<T>, (cols * 32 + 255) / 256, 256, 0, s, W, ldw, rows, cols, nrm)));
+        HEFF_CUDA((launch_chained(col_order_kernel, (cols + 127) / 128, 128, 0, s, nrm, cols, ord)));
         return HEFF_OK;
     };
     // Preconditioned from 17 columns on, and whenever the rows are many: measured on real 32 x 32 matrices, 0.39 ms with and
@@ -1220,25 +1212,20 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     if(wide && (precond || !whole)) {
         T *dst = precond ? Z : G;
         HEFF_CUDA(cudaMemsetAsync(dst, 0, sizeof(T) * (size_t)ldg * npad, s));
-        adjoint_kernel<T, false><<<dim3((unsigned)cdiv(N, 32), (unsigned)cdiv(M, 32)), 256, 0, s>>>(A, lda, (int)m, (int)n, dst, ldg, M, N);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(adjoint_kernel<T, false>, dim3((unsigned)cdiv(N, 32), (unsigned)cdiv(M, 32)), 256, 0, s, A, lda, (int)m, (int)n, dst, ldg, M, N)));
         src = dst, lds = ldg;
     }
     if(precond) {
         // G = A or A^H with the columns by descending norm: the factors of a matrix whose columns differ by orders of
         // magnitude keep each column's own relative accuracy, and zero columns come last
         HEFF_TRY(norms_order(src, lds, M, N, sig0, cord));
-        copy_pad_kernel<T><<<g1(ldg * npad), 256, 0, s>>>(src, lds, M, N, G, ldg, npad, cord);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(copy_pad_kernel<T>, g1(ldg * npad), 256, 0, s, src, lds, M, N, G, ldg, npad, cord)));
         HEFF_TRY(qr_factor<T>(G, ldg, M, N, T1, s));
-        adjoint_kernel<T, true><<<dim3((unsigned)(npad / 32), (unsigned)(npad / 32)), 256, 0, s>>>(G, ldg, N, N, X, npad, npad, npad);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, dim3((unsigned)(npad / 32), (unsigned)(npad / 32)), 256, 0, s, G, ldg, N, N, X, npad, npad, npad)));
         HEFF_TRY(qr_factor<T>(X, npad, N, N, T2, s));
-        adjoint_kernel<T, true><<<dim3((unsigned)(npad / 32), (unsigned)(npad / 32)), 256, 0, s>>>(X, npad, N, N, Y, npad, npad, npad);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, dim3((unsigned)(npad / 32), (unsigned)(npad / 32)), 256, 0, s, X, npad, N, N, Y, npad, npad, npad)));
     } else if(!wide && !whole) {
-        copy_pad_kernel<T><<<g1(ldg * npad), 256, 0, s>>>(src, lds, M, N, G, ldg, npad, nullptr);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(copy_pad_kernel<T>, g1(ldg * npad), 256, 0, s, src, lds, M, N, G, ldg, npad, nullptr)));
     }
     const int B = npad / JB;  // even
     // off-diagonal tolerance just above the rounding noise of a length-m dot product
@@ -1251,13 +1238,11 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
         const int64_t ldf  = precond ? ldw : lda;
         const int     adj  = !precond && wide;
         if(npad == 32)
-            jacobi_whole_kernel<T, 32><<<1, jw_thr(32), jacobi_whole_bytes<T, 32>(), s>>>(from, ldf, adj, W, ldw, rows, N, V, tol, JOUTER, sig, drot);
+            HEFF_CUDA((launch_chained(jacobi_whole_kernel<T, 32>, 1, jw_thr(32), jacobi_whole_bytes<T, 32>(), s, from, ldf, adj, W, ldw, rows, N, V, tol, JOUTER, sig, drot)));
         else
-            jacobi_whole_kernel<T, 64><<<1, jw_thr(64), jacobi_whole_bytes<T, 64>(), s>>>(from, ldf, adj, W, ldw, rows, N, V, tol, JOUTER, sig, drot);
-        HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(jacobi_whole_kernel<T, 64>, 1, jw_thr(64), jacobi_whole_bytes<T, 64>(), s, from, ldf, adj, W, ldw, rows, N, V, tol, JOUTER, sig, drot)));
     } else {
-        eye_kernel<T><<<g1((int64_t)npad * npad), 256, 0, s>>>(V, npad, npad);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(eye_kernel<T>, g1((int64_t)npad * npad), 256, 0, s, V, npad, npad)));
         // Norm-ordered blocks (the block form of de Rijk's pivoting in LAPACK's ?gesvj): before every sweep the
         // columns are ordered by norm and blocks are formed from neighbours, so clusters of close singular values
         // meet inside one pair block.  CTAs per pair: enough to fill the SMs with one wave (the pairs of a round are only
@@ -1269,25 +1254,8 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
             HEFF_TRY(norms_order(W, ldw, rows, npad, sig, cmap));
             HEFF_CUDA(cudaMemsetAsync(dmax, 0, 2 * sizeof(double), s));
             for(int r = 0; r < B - 1; r++) {
-                if(CL == 1) {
-                    jacobi_round_kernel<T><<<B / 2, JTHR, jacobi_round_bytes<T>(), s>>>(W, ldw, rows, V, npad, npad, B, r, tol, floor_abs, cmap, dmax, drot, 1);
-                    HEFF_LAUNCH_CHECK();
-                } else {
-                    cudaLaunchConfig_t  lc = {};
-                    cudaLaunchAttribute at[1];
-                    at[0].id               = cudaLaunchAttributeClusterDimension;
-                    at[0].val.clusterDim.x = (unsigned)CL;
-                    at[0].val.clusterDim.y = 1;
-                    at[0].val.clusterDim.z = 1;
-                    lc.gridDim             = dim3((unsigned)(B / 2 * CL));
-                    lc.blockDim            = dim3(JTHR);
-                    lc.dynamicSmemBytes    = jacobi_round_bytes<T>();
-                    lc.stream              = s;
-                    lc.attrs               = at;
-                    lc.numAttrs            = 1;
-                    HEFF_CUDA(cudaLaunchKernelEx(&lc, jacobi_round_kernel<T>, W, ldw, rows, V, (int64_t)npad, (int)npad, B, r, tol, floor_abs,
-                                                 (const int *)cmap, dmax, drot, CL));
-                }
+                HEFF_CUDA((launch_chained_cluster((unsigned)CL, jacobi_round_kernel<T>, B / 2 * CL, JTHR, jacobi_round_bytes<T>(), s, W, ldw, rows, V, npad,
+                                                  npad, B, r, tol, floor_abs, cmap, dmax, drot, CL)));
             }
             struct {
                 double gmax;
@@ -1298,8 +1266,7 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
             if(st.rot == 0) break;
             floor_abs = (double)rows * eps * eps * st.gmax;
         }
-        col_norms_kernel<T><<<(npad * 32 + 255) / 256, 256, 0, s>>>(W, ldw, rows, npad, sig);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(col_norms_kernel<T>, (npad * 32 + 255) / 256, 256, 0, s, W, ldw, rows, npad, sig)));
     }
     HEFF_CUDA(cudaMemcpyAsync(host.data(), sig, sizeof(double) * host.size(), cudaMemcpyDeviceToHost, s));
     HEFF_CUDA(cudaStreamSynchronize(s));
@@ -1331,23 +1298,20 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     const int kk = (int)r, gr = g1((int64_t)(M + N) * r);
     if(!precond) {
         if(!wide)
-            take_columns_kernel<T, false, true><<<gr, 256, 0, s>>>(W, ldw, rows, V, npad, N, perm, sig, kk, S, U, M, M, VT, 0);
+            HEFF_CUDA((launch_chained(take_columns_kernel<T, false, true>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, U, M, M, VT, 0)));
         else
-            take_columns_kernel<T, true, false><<<gr, 256, 0, s>>>(W, ldw, rows, V, npad, N, perm, sig, kk, S, VT, 0, M, U, N);
-        HEFF_LAUNCH_CHECK();
+            HEFF_CUDA((launch_chained(take_columns_kernel<T, true, false>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, VT, 0, M, U, N)));
     } else {
         T            *left = wide ? Z : U;
         const int64_t ldl  = wide ? ldg : M;
-        take_columns_kernel<T, false, false><<<gr, 256, 0, s>>>(W, ldw, rows, V, npad, N, perm, sig, kk, S, left, ldl, M, R, npad);
-        HEFF_LAUNCH_CHECK();
+        HEFF_CUDA((launch_chained(take_columns_kernel<T, false, false>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, left, ldl, M, R, npad)));
         HEFF_TRY(qr_apply_q<T>(G, ldg, M, N, T1, left, ldl, kk, s));
         HEFF_TRY(qr_apply_q<T>(X, npad, N, N, T2, R, npad, kk, s));
         if(!wide) {
-            adjoint_rows_kernel<T><<<g1((int64_t)N * r), 256, 0, s>>>(R, npad, N, kk, cord, VT);
+            HEFF_CUDA((launch_chained(adjoint_rows_kernel<T>, g1((int64_t)N * r), 256, 0, s, R, npad, N, kk, cord, VT)));
         } else {  // A^H = left S right^H: U = right, VT = left^H
-            scatter_rows_kernel<T><<<g1((int64_t)N * r), 256, 0, s>>>(R, npad, N, kk, cord, U, m);
-            HEFF_LAUNCH_CHECK();
-            adjoint_rows_kernel<T><<<g1((int64_t)M * r), 256, 0, s>>>(left, ldl, M, kk, nullptr, VT);
+            HEFF_CUDA((launch_chained(scatter_rows_kernel<T>, g1((int64_t)N * r), 256, 0, s, R, npad, N, kk, cord, U, m)));
+            HEFF_CUDA((launch_chained(adjoint_rows_kernel<T>, g1((int64_t)M * r), 256, 0, s, left, ldl, M, kk, nullptr, VT)));
         }
         HEFF_LAUNCH_CHECK();
     }
@@ -1367,6 +1331,7 @@ int svd_truncated(const double2 *A, int64_t lda, int64_t m, int64_t n, int64_t r
 // theta [dL*dR, chiL, chiR] -> A[(s1 + dL a), (s2 + dR b)] = theta[s1 + dL s2, a, b]   (svd.h:217 reshape+shuffle)
 template<class T>
 __global__ void schmidt_pack_kernel(const T *__restrict__ th, T *__restrict__ A, int64_t dL, int64_t dR, int64_t cL, int64_t cR) {
+    grid_wait();
     const int64_t m = dL * cL, tot = m * dR * cR;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = e % m, col = e / m;
@@ -1378,6 +1343,7 @@ __global__ void schmidt_pack_kernel(const T *__restrict__ th, T *__restrict__ A,
 template<class T>
 __global__ void schmidt_unpack_kernel(const T *__restrict__ VT, T *__restrict__ Vout, double *__restrict__ S, double inv_norm, int64_t k, int64_t dR,
                                       int64_t cR) {
+    grid_wait();
     const int64_t tot = k * dR * cR;
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s2 = e % dR, r = e / dR, i = r % k, b = r / k;
@@ -1400,8 +1366,7 @@ static int schmidt_split_t(const T *theta, int64_t dL, int64_t dR, int64_t cL, i
     T            *VT   = A + (m * n + 31) / 32 * 32;
     const int64_t kmax = std::min(std::min(m, n), rank_max > 0 ? rank_max : INT64_MAX);
     void         *jscr = VT + (kmax * n + 31) / 32 * 32;
-    schmidt_pack_kernel<T><<<g1(m * n), 256, 0, s>>>(theta, A, dL, dR, cL, cR);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(schmidt_pack_kernel<T>, g1(m * n), 256, 0, s, theta, A, dL, dR, cL, cR)));
     HEFF_TRY(svd_truncated_t<T>(A, m, m, n, rank_max, trunc_lim, U, S, VT, rank, trunc_err, jscr, nullptr, s));
     std::vector<double> hs(*rank);
     HEFF_CUDA(cudaMemcpyAsync(hs.data(), S, sizeof(double) * (*rank), cudaMemcpyDeviceToHost, s));
@@ -1409,8 +1374,7 @@ static int schmidt_split_t(const T *theta, int64_t dL, int64_t dR, int64_t cL, i
     double nrm = 0;
     for(double v : hs) nrm += v * v;
     nrm = std::sqrt(nrm);
-    schmidt_unpack_kernel<T><<<g1((*rank) * n), 256, 0, s>>>(VT, V, S, nrm > 0 ? 1.0 / nrm : 1.0, *rank, dR, cR);
-    HEFF_LAUNCH_CHECK();
+    HEFF_CUDA((launch_chained(schmidt_unpack_kernel<T>, g1((*rank) * n), 256, 0, s, VT, V, S, nrm > 0 ? 1.0 / nrm : 1.0, *rank, dR, cR)));
     return HEFF_OK;
 }
 

@@ -83,6 +83,7 @@ __device__ void build_wlist_serial(const T *W, int DL, int DR, int S, unsigned c
 }
 template<class T>
 __global__ void wlist_global_kernel(const T *W, int DL, int DR, int S, unsigned char *out) {
+    grid_wait();
     if(threadIdx.x == 0 && blockIdx.x == 0) build_wlist_serial(W, DL, DR, S, out);
 }
 // Views of a list block laid out as above.
