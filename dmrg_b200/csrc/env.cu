@@ -17,15 +17,6 @@ namespace heff {
 
 __device__ __forceinline__ double conj_s(double v) { return v; }
 __device__ __forceinline__ double2 conj_s(double2 v) { return make_double2(v.x, -v.y); }
-__device__ __forceinline__ double fma_e(double w, double v, double acc) { return fma(w, v, acc); }
-__device__ __forceinline__ double2 fma_e(double2 w, double2 v, double2 acc) {
-    return make_double2(fma(w.x, v.x, fma(-w.y, v.y, acc.x)), fma(w.x, v.y, fma(w.y, v.x, acc.y)));
-}
-__device__ __forceinline__ bool nz(double w) { return w != 0.0; }
-__device__ __forceinline__ bool nz(double2 w) { return w.x != 0.0 || w.y != 0.0; }
-__device__ __forceinline__ void setz(double &v) { v = 0.0; }
-__device__ __forceinline__ void setz(double2 &v) { v = make_double2(0.0, 0.0); }
-
 // Mc[a' + cL*(s' + d*b')] = conj(M[s' + d*(a' + cL*b')])
 template<class T>
 __global__ void env_prep_L(const T *__restrict__ M, T *__restrict__ Mc, int64_t d, int64_t cL, int64_t n) {
@@ -46,37 +37,21 @@ __global__ void env_prep_R(const T *__restrict__ M, T *__restrict__ Mc, T *__res
     }
 }
 
-// Mix of both sides. One thread per (p, q): p runs over the contiguous index of X (a for L, b for R),
-// q over the other point index (b' for L, a' for R).
+// Mix of both sides (mpo_mix): p runs over the contiguous index of X (a for L, b for R), q over the other point index (b' for
+// L, a' for R).
 //   in[k, s'] = X[p + P*(s' + d*q) + P*d*Q*k]      (k = m for L, n for R)
 //   out[j, s] = Y[s + d*p + d*P*(q + Q*j)]         (j = n for L, m for R)
 //   L: out[n,s] = sum_{m,s'} W[m,n,s,s'] in[m,s'];   R: out[m,s] = sum_{n,s'} W[m,n,s,s'] in[n,s']
-template<class T, bool LEFT>
-__global__ void env_mix_kernel(const T *__restrict__ X, T *__restrict__ Y, const T *__restrict__ W, int d, int P, int Q, int DL, int DR) {
-    grid_wait();
-    extern __shared__ __align__(16) unsigned char env_smem[];
-    T        *sW = reinterpret_cast<T *>(env_smem);
-    const int nW = DL * DR * d * d;
-    for(int i = threadIdx.x; i < nW; i += blockDim.x) sW[i] = W[i];
-    __syncthreads();
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int q = blockIdx.y;
-    if(p >= P) return;
-    const int     Kin = LEFT ? DL : DR, Kout = LEFT ? DR : DL;
-    const int64_t PdQ = (int64_t)P * d * Q;
-    for(int j = 0; j < Kout; j++) {
-        for(int s = 0; s < d; s++) {
-            T acc;
-            setz(acc);
-            for(int k = 0; k < Kin; k++)
-                for(int sp = 0; sp < d; sp++) {
-                    const int m = LEFT ? k : j, n = LEFT ? j : k;
-                    const T   w = sW[m + DL * (n + DR * (s + d * sp))];
-                    if(nz(w)) acc = fma_e(w, X[p + (int64_t)P * (sp + (int64_t)d * q) + PdQ * k], acc);
-                }
-            Y[s + (int64_t)d * p + (int64_t)d * P * (q + (int64_t)Q * j)] = acc;
-        }
-    }
+template<bool CPLX>
+static int env_mix(bool left, const typename Scalar<CPLX>::T *X, typename Scalar<CPLX>::T *Y, const typename Scalar<CPLX>::T *W, int64_t d, int64_t P,
+                   int64_t Q, int64_t DL, int64_t DR, cudaStream_t s) {
+    MixArgs a{};
+    a.in = X, a.out = Y, a.W = W;
+    a.K = (int)(left ? DL : DR), a.J = (int)(left ? DR : DL), a.S = (int)d, a.P = (int)P, a.Q = (int)Q, a.q0 = 0, a.nq = (int)Q;
+    a.in_k = P * d * Q, a.in_s = P, a.in_q = P * d;
+    a.w_k = left ? 1 : (int)DL, a.w_j = left ? (int)DL : 1, a.w_s = (int)(DL * DR * d), a.w_so = (int)(DL * DR);
+    a.s_fastest = true;
+    return mpo_mix<CPLX>(a, s);
 }
 
 static int grid1(int64_t n) {
@@ -126,7 +101,6 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
     T            *M2  = Mc + pad(nM);
     T            *X   = M2 + pad(nM);
     T            *Y   = X + pad(Dm * nM);
-    const size_t  wsm = sizeof(T) * (size_t)(DL * DR * d * d);
     if(side == 0) {
         HEFF_CUDA((launch_chained(env_prep_L<T>, grid1(nM), 256, 0, s, M, Mc, d, cL, nM)));
         GemmArgs g{};
@@ -137,8 +111,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
         HEFF_TRY(gemm_f64<CPLX>(false, false, g, s));
         if(cR > 65535) return HEFF_BAD_SHAPE;
-        dim3 grid((unsigned)cdiv(cL, 128), (unsigned)cR);
-        HEFF_CUDA((launch_chained(env_mix_kernel<T, true>, grid, 128, wsm, s, X, Y, W, (int)d, (int)cL, (int)cR, (int)DL, (int)DR)));
+        HEFF_TRY(env_mix<CPLX>(true, X, Y, W, d, cL, cR, DL, DR, s));
         GemmArgs h{};
         h.M = (int)cR, h.N = (int)(cR * DR), h.K = (int)(d * cL), h.batch = 1;
         h.A = M, h.lda = d * cL, h.B = Y, h.ldb = d * cL, h.C = out, h.ldc = cR;
@@ -155,8 +128,7 @@ int env_update(int side, typename Scalar<CPLX>::T *out, const typename Scalar<CP
         g.alpha = make_double2(1, 0), g.beta = make_double2(0, 0);
         HEFF_TRY(gemm_f64<CPLX>(false, true, g, s));
         if(cL > 65535) return HEFF_BAD_SHAPE;
-        dim3 grid((unsigned)cdiv(cR, 128), (unsigned)cL);
-        HEFF_CUDA((launch_chained(env_mix_kernel<T, false>, grid, 128, wsm, s, X, Y, W, (int)d, (int)cR, (int)cL, (int)DL, (int)DR)));
+        HEFF_TRY(env_mix<CPLX>(false, X, Y, W, d, cR, cL, DL, DR, s));
         GemmArgs h{};
         h.M = (int)cL, h.N = (int)(cL * DL), h.K = (int)(d * cR), h.batch = 1;
         h.A = M2, h.lda = d * cR, h.B = Y, h.ldb = d * cR, h.C = out, h.ldc = cL;

@@ -70,55 +70,247 @@ __device__ __forceinline__ double2 fma_s(double2 w, double2 v, double2 acc) {
 __device__ __forceinline__ void zero(double &v) { v = 0.0; }
 __device__ __forceinline__ void zero(double2 &v) { v = make_double2(0.0, 0.0); }
 
-// T2[(s' + S a') + S cL (b + cR n)] = sum_{m,s} W[m + DL(n + DR(s + S s'))] T1[(a' + cL m) + cL DL (s + S b)]
-// One CTA: 128 consecutive a' at one b.  W, its nonzero list (wlist.cuh) and the CTA's T1 column block are
-// staged in shared memory; each output runs only over the nonzero MPO entries.
-constexpr int MIX_THREADS = 128;
+// MPO mix (MixArgs, matvec.cuh) on the FP64 tensor pipe: at 16 points of a warp, out (16 x J S) = in (16 x K S) W.  The
+// dense product costs less than walking W's nonzero entries (~20 % in spin chains) with a shared-memory load or two per
+// multiply-add: 6 DMMAs per 16 points for the two-site Ising MPO (D = 3), 45 for its square, and the kernel stays bound by
+// HBM for large tensors and by its two dependent memory latencies for small ones.  W is laid out once per CTA as DMMA
+// fragments; a CTA owns TP consecutive points p and walks q in steps of gridDim.y with the next tile in flight.  Two
+// accumulator columns are two consecutive s', so eight points' stores of one (j, s') pair fill whole sectors.
+// A zero weight must not touch its input: the reference skips zero entries, and 0 * inf would not.  A warp that meets a
+// non-finite input computes its points entry by entry instead (mix_skip).
+// us before / after: chi = 16 real D = 3 10.6 / 5.2, chi = 1024 complex D = 3 114 / 89 (HBM floor 62), real D = 9 367 x 251
+// 53 / 26, environment real D = 9 640 x 517 165 / 43.
 template<class T>
-__global__ void __launch_bounds__(MIX_THREADS) mix_kernel(const T *__restrict__ T1, T *__restrict__ T2, const T *__restrict__ W, int S, int cL,
-                                                         int cR, int DL, int DR, int b0) {
-    grid_wait();
-    extern __shared__ __align__(16) unsigned char mix_smem[];
-    T        *sW  = reinterpret_cast<T *>(mix_smem);
-    const int nW  = DL * DR * S * S;
-    T        *sIn = sW + nW;
-    unsigned char *lmem = reinterpret_cast<unsigned char *>(sIn + (size_t)DL * S * MIX_THREADS);
-    for(int i = threadIdx.x; i < nW; i += blockDim.x) sW[i] = W[i];
-    const int     b   = b0 + blockIdx.y;  // columns b0 .. b0 + gridDim.y - 1
-    const int     ap  = blockIdx.x * MIX_THREADS + threadIdx.x;
-    const bool    act = ap < cL;
-    const int64_t cLD = (int64_t)cL * DL;
-    // 8 loads in flight per thread before their shared-memory stores (slot ms = m*S + s)
-    const int NP = DL * S;
-    for(int ms0 = 0; ms0 < NP; ms0 += 8) {
-        T v[8];
-#pragma unroll
-        for(int u = 0; u < 8; u++) {
-            const int ms = ms0 + u, m = ms / S, s = ms % S;
-            zero(v[u]);
-            if(act && ms < NP) v[u] = T1[(ap + (int64_t)cL * m) + cLD * (s + (int64_t)S * b)];
+__device__ __noinline__ void mix_skip(const MixArgs &a, const T *tile, int pitch, int p, int q, int o0, int o1) {
+    const int S = a.S, NI = a.K * S;
+    const T  *W = reinterpret_cast<const T *>(a.W);
+    for(int o = o0; o < o1; o++) {
+        const int j = o / S, so = o - j * S;
+        T         acc;
+        zero(acc);
+        for(int i = 0; i < NI; i++) {
+            const int k = a.s_fastest ? i / S : i % a.K, s = a.s_fastest ? i % S : i / a.K;
+            const T   w = W[(int64_t)a.w_k * k + (int64_t)a.w_j * j + (int64_t)a.w_s * s + (int64_t)a.w_so * so];
+            if(!is_zero(w)) acc = fma_s(w, tile[(k * S + s) * pitch], acc);
         }
-#pragma unroll
-        for(int u = 0; u < 8; u++)
-            if(ms0 + u < NP) sIn[(ms0 + u) * MIX_THREADS + threadIdx.x] = v[u];
-    }
-    __syncthreads();
-    int   *off;
-    short *idx;
-    T     *wv;
-    build_wlist(sW, DL, DR, S, lmem, off, idx, wv);
-    if(!act) return;
-    for(int n = 0; n < DR; n++) {
-        T *out = T2 + ((int64_t)S * ap) + (int64_t)S * cL * (b + (int64_t)cR * n);
-        for(int sp = 0; sp < S; sp++) {
-            const int o = n * S + sp;
-            T         acc;
-            zero(acc);
-            for(int e = off[o]; e < off[o + 1]; e++) acc = fma_s(wv[e], sIn[idx[e] * MIX_THREADS + threadIdx.x], acc);
-            out[sp] = acc;
-        }
+        reinterpret_cast<T *>(a.out)[so + (int64_t)S * (p + (int64_t)a.P * (q + (int64_t)a.Q * j))] = acc;
     }
 }
+
+__device__ __forceinline__ bool non_finite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool non_finite(double2 v) { return non_finite(v.x) || non_finite(v.y); }
+
+template<class T, int TP>
+struct MixTile {
+    static constexpr bool CX    = sizeof(T) == 16;
+    static constexpr int  THR   = 2 * TP;                // one warp per 16 points
+    static constexpr int  PITCH = TP + (CX ? 2 : 4);     // conflict-free fragment loads
+};
+template<class T, int TP, int NTC>
+__global__ void __launch_bounds__(2 * TP) mix_dense_kernel(const MixArgs a) {
+    grid_wait();
+    using MT = MixTile<T, TP>;
+    constexpr bool CX = MT::CX;
+    constexpr int  THR = MT::THR, WARPS = THR / 32, PITCH = MT::PITCH;
+    extern __shared__ __align__(16) unsigned char mix_smem[];
+    const int    S = a.S, NI = a.K * S, NO = a.J * S, KS = (NI + 3) / 4, NT = (NO + 7) / 8;
+    T           *tile = reinterpret_cast<T *>(mix_smem);                 // a.bufs tiles of 4 KS x PITCH (rows past NI are zero)
+    T           *frag = tile + (size_t)a.bufs * 4 * KS * PITCH;          // (ks, nt, lane)
+    const T     *in   = reinterpret_cast<const T *>(a.in), *W = reinterpret_cast<const T *>(a.W);
+    T           *out  = reinterpret_cast<T *>(a.out);
+    const int    tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int    p0 = blockIdx.x * TP, np = min(TP, a.P - p0);
+    auto load = [&](int q, int buf) {
+        T       *dst = tile + (size_t)buf * 4 * KS * PITCH;
+        const T *src = in + p0 + a.in_q * q;
+        for(int i = warp; i < 4 * KS; i += WARPS) {
+            const int  k = i / S, s = i - k * S;
+            const bool row = i < NI;
+            const T   *r   = src + a.in_k * k + a.in_s * s;
+            if(CX || a.vec) {
+                constexpr int E = CX ? 1 : 2;
+                for(int p = lane * E; p < TP; p += 32 * E) cp_async<16>(smem_u32(dst + i * PITCH + p), row && p < np ? r + p : in, row && p < np);
+            } else {
+                for(int p = lane; p < TP; p += 32) cp_async<(int)sizeof(T)>(smem_u32(dst + i * PITCH + p), row && p < np ? r + p : in, row && p < np);
+            }
+        }
+        cp_async_commit();
+    };
+    int q = a.q0 + (int)blockIdx.y;
+    load(q, 0);
+    bool wim = false;  // W has an imaginary part
+    for(int e = tid; e < KS * NT * 32; e += THR) {
+        const int f = e >> 5, i = (f / NT) * 4 + (e & 3), o = (f % NT) * 8 + ((e & 31) >> 2);
+        T         v;
+        zero(v);
+        if(i < NI && o < NO) {
+            const int k = i / S, s = i - k * S, j = o / S, so = o - j * S;
+            v = W[(int64_t)a.w_k * k + (int64_t)a.w_j * j + (int64_t)a.w_s * s + (int64_t)a.w_so * so];
+        }
+        frag[e] = v;
+        if constexpr(CX) wim = wim || v.y != 0.0;
+    }
+    if constexpr(CX) wim = __syncthreads_or(wim) != 0;
+    const int     pw = warp * 16;                       // this warp's points of the tile
+    const int64_t jstep = (int64_t)S * a.P * a.Q;
+    for(int buf = 0; q < a.q0 + a.nq; q += (int)gridDim.y, buf ^= a.bufs - 1) {
+        const int qn = q + (int)gridDim.y;
+        if(a.bufs == 2) {
+            if(qn < a.q0 + a.nq)
+                load(qn, buf ^ 1);
+            else
+                cp_async_commit();
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        const T *x   = tile + (size_t)buf * 4 * KS * PITCH + pw;
+        bool     bad = false;
+        if(pw < np) {
+            for(int n0 = 0; n0 < NT; n0 += NTC) {
+                double re[NTC][4], im[CX ? NTC : 1][4];
+#pragma unroll
+                for(int n = 0; n < NTC; n++)
+#pragma unroll
+                    for(int u = 0; u < 4; u++) {
+                        re[n][u] = 0.0;
+                        if constexpr(CX) im[n][u] = 0.0;
+                    }
+#pragma unroll 2
+                for(int ks = 0; ks < KS; ks++) {
+                    const T a0 = x[(4 * ks + t) * PITCH + g], a1 = x[(4 * ks + t) * PITCH + g + 8];
+                    bad        = bad || non_finite(a0) || non_finite(a1);
+                    const T *fr = frag + (size_t)(ks * NT + n0) * 32 + lane;
+#pragma unroll
+                    for(int n = 0; n < NTC; n++)
+                        if(n0 + n < NT) {
+                            const T b = fr[n * 32];
+                            if constexpr(!CX) {
+                                dmma(re[n], a0, a1, b);
+                            } else {
+                                dmma(re[n], a0.x, a1.x, b.x);
+                                dmma(im[n], a0.y, a1.y, b.x);
+                                if(wim) {
+                                    dmma(re[n], -a0.y, -a1.y, b.y);
+                                    dmma(im[n], a0.x, a1.x, b.y);
+                                }
+                            }
+                        }
+                }
+                if(__any_sync(0xffffffffu, bad)) break;
+#pragma unroll
+                for(int n = 0; n < NTC; n++) {
+                    const int o = (n0 + n) * 8 + 2 * t;
+                    if(o >= NO) continue;
+                    const int j = o / S, so = o - j * S;
+#pragma unroll
+                    for(int h = 0; h < 2; h++) {
+                        const int p = pw + g + 8 * h;
+                        if(p >= np) continue;
+                        T *dst = out + so + jstep * j + (int64_t)S * (p0 + p + (int64_t)a.P * q);
+                        T  v0, v1;
+                        if constexpr(!CX)
+                            v0 = re[n][2 * h], v1 = re[n][2 * h + 1];
+                        else
+                            v0 = make_double2(re[n][2 * h], im[n][2 * h]), v1 = make_double2(re[n][2 * h + 1], im[n][2 * h + 1]);
+                        if(!CX && a.pairs) {
+                            if constexpr(!CX) *reinterpret_cast<double2 *>(dst) = make_double2(v0, v1);
+                        } else {
+                            dst[0] = v0;
+                            if(o + 1 < NO) (so + 1 < S ? dst + 1 : dst - so + jstep)[0] = v1;
+                        }
+                    }
+                }
+            }
+            if(__any_sync(0xffffffffu, bad)) {  // lanes 0..15 and 16..31 take half of the outputs each, a point per lane
+                const int p = pw + (lane & 15), half = (NO + 1) / 2;
+                if(p < np) mix_skip<T>(a, x + (lane & 15), PITCH, p0 + p, q, lane < 16 ? 0 : half, lane < 16 ? half : NO);
+            }
+        }
+        __syncthreads();  // the tile has been read
+        if(a.bufs == 1 && qn < a.q0 + a.nq) load(qn, 0);
+    }
+}
+
+// Entry by entry from global memory: MPO bonds whose dense product would not pay (more than MIX_DENSE fragments) or whose
+// tiles do not fit.  One thread per point, W's entries by uniform loads.
+template<class T>
+__global__ void __launch_bounds__(128) mix_entry_kernel(const MixArgs a) {
+    grid_wait();
+    const int S = a.S, NI = a.K * S;
+    const T  *W = reinterpret_cast<const T *>(a.W);
+    for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)a.P * a.nq; e += (int64_t)gridDim.x * blockDim.x) {
+        const int p = (int)(e % a.P), q = a.q0 + (int)(e / a.P);
+        const T  *x = reinterpret_cast<const T *>(a.in) + p + a.in_q * q;
+        T        *o = reinterpret_cast<T *>(a.out) + (int64_t)S * (p + (int64_t)a.P * q);
+        for(int j = 0; j < a.J; j++)
+            for(int so = 0; so < S; so++) {
+                T acc;
+                zero(acc);
+                for(int i = 0; i < NI; i++) {
+                    const int k = a.s_fastest ? i / S : i % a.K, s = a.s_fastest ? i % S : i / a.K;
+                    const T   w = __ldg(W + (int64_t)a.w_k * k + (int64_t)a.w_j * j + (int64_t)a.w_s * s + (int64_t)a.w_so * so);
+                    if(!is_zero(w)) acc = fma_s(w, x[a.in_k * k + a.in_s * s], acc);
+                }
+                o[so + (int64_t)S * a.P * a.Q * j] = acc;
+            }
+    }
+}
+
+template<class T, int TP>
+static size_t mix_bytes(const MixArgs &a, int bufs) {
+    const size_t KS = (size_t)cdiv((int64_t)a.K * a.S, 4), NT = (size_t)cdiv((int64_t)a.J * a.S, 8);
+    return sizeof(T) * (bufs * 4 * KS * MixTile<T, TP>::PITCH + KS * NT * 32);
+}
+constexpr size_t MIX_SMEM = 200 * 1024;
+template<class T, int TP, int NTC>
+static int mix_launch(const MixArgs &a, cudaStream_t s) {
+    const size_t smem = mix_bytes<T, TP>(a, a.bufs);
+    static int   attr_done[64] = {0};
+    int          dev           = 0;
+    HEFF_CUDA(cudaGetDevice(&dev));
+    if(dev < 0 || dev >= 64 || !attr_done[dev]) {
+        HEFF_CUDA(cudaFuncSetAttribute(mix_dense_kernel<T, TP, NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MIX_SMEM));
+        if(dev >= 0 && dev < 64) attr_done[dev] = 1;
+    }
+    // about as many CTAs as the device holds; each then lays W out once for several q
+    const int64_t tx  = cdiv(a.P, TP);
+    const int64_t occ = std::max<int64_t>(1, std::min<int64_t>(1024 / MixTile<T, TP>::THR, (int64_t)(224 * 1024 / (smem + 1024))));
+    const int64_t ny  = std::min<int64_t>(a.nq, std::max<int64_t>(1, (int64_t)device_sm_count() * occ / tx));
+    HEFF_CUDA((launch_chained(mix_dense_kernel<T, TP, NTC>, dim3((unsigned)tx, (unsigned)ny), MixTile<T, TP>::THR, smem, s, a)));
+    return HEFF_OK;
+}
+// Two tiles in flight where two such CTAs fit an SM.
+template<class T, int TP>
+static int mix_tiles(MixArgs a, cudaStream_t s) {
+    a.bufs = mix_bytes<T, TP>(a, 2) <= 110 * 1024 ? 2 : 1;
+    return cdiv((int64_t)a.J * a.S, 8) <= 2 ? mix_launch<T, TP, 2>(a, s) : mix_launch<T, TP, 5>(a, s);
+}
+// Points per tile: 128, fewer while that leaves SMs without a CTA or the tile does not fit.
+constexpr int64_t MIX_DENSE = 64;  // DMMA fragments of W up to which the dense product is taken (D = 9, S = 4 has 45)
+template<bool CPLX>
+int mpo_mix(MixArgs a, cudaStream_t s) {
+    using T = typename Scalar<CPLX>::T;
+    if(a.nq <= 0 || a.P <= 0) return HEFF_OK;
+    a.pairs = !CPLX && a.S % 2 == 0 && ((uintptr_t)a.out & 15u) == 0;
+    a.vec   = !CPLX && ((uintptr_t)a.in & 15u) == 0 && a.P % 2 == 0 && a.in_k % 2 == 0 && a.in_s % 2 == 0 && a.in_q % 2 == 0;
+    const int64_t frags = cdiv((int64_t)a.K * a.S, 4) * cdiv((int64_t)a.J * a.S, 8);
+    if(frags > MIX_DENSE || mix_bytes<T, 32>(a, 1) > MIX_SMEM) {
+        const int64_t n = (int64_t)a.P * a.nq, g = std::min<int64_t>(cdiv(n, 128), (int64_t)device_sm_count() * 16);
+        HEFF_CUDA((launch_chained(mix_entry_kernel<T>, (unsigned)g, 128, 0, s, a)));
+        return HEFF_OK;
+    }
+    auto padded = [&](int tp) { return cdiv(a.P, tp) * tp; };
+    int  TP     = 128;
+    if(cdiv(a.P, 128) * a.nq < 2 * device_sm_count() || mix_bytes<T, 128>(a, 1) > MIX_SMEM || 16 * padded(128) > 17 * padded(64)) TP = 64;
+    if(TP == 64 && (cdiv(a.P, 64) * a.nq < 2 * device_sm_count() || mix_bytes<T, 64>(a, 1) > MIX_SMEM || 16 * padded(64) > 17 * padded(32))) TP = 32;
+    if(TP == 128) return mix_tiles<T, 128>(a, s);
+    if(TP == 64) return mix_tiles<T, 64>(a, s);
+    return mix_tiles<T, 32>(a, s);
+}
+template int mpo_mix<false>(MixArgs, cudaStream_t);
+template int mpo_mix<true>(MixArgs, cudaStream_t);
 
 static int grid_1d(int64_t n) {
     int64_t g = (n + 255) / 256;
@@ -133,26 +325,22 @@ int permute_R(const typename Scalar<CPLX>::T *R, typename Scalar<CPLX>::T *Rp, c
     return HEFF_OK;
 }
 
+// T2[(s' + S a') + S cL (b + cR n)] = sum_{m,s} W[m + DL(n + DR(s + S s'))] T1[(a' + cL m) + cL DL (s + S b)], b0 <= b < b0 + nb
 template<bool CPLX>
 static int launch_mix(const MatvecDims &d, const typename Scalar<CPLX>::T *T1, typename Scalar<CPLX>::T *T2, const typename Scalar<CPLX>::T *W,
                       cudaStream_t s, int64_t b0 = 0, int64_t nb = -1) {
-    using T           = typename Scalar<CPLX>::T;
-    const size_t smem = sizeof(T) * ((size_t)d.DL * d.DR * d.S * d.S + (size_t)d.DL * d.S * MIX_THREADS) +
-                        wlist_bytes((int)d.DL, (int)d.DR, (int)d.S, sizeof(T));
-    if(smem > 200 * 1024) return HEFF_BAD_SHAPE;
-    static int attr_done[64] = {0};
-    int        dev           = 0;
-    HEFF_CUDA(cudaGetDevice(&dev));
-    if(dev < 0 || dev >= 64 || !attr_done[dev]) {
-        HEFF_CUDA(cudaFuncSetAttribute(mix_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        if(dev >= 0 && dev < 64) attr_done[dev] = 1;
-    }
+    using T = typename Scalar<CPLX>::T;
+    // limit on the MPO's size
+    const size_t need = sizeof(T) * ((size_t)d.DL * d.DR * d.S * d.S + (size_t)d.DL * d.S * 128) + wlist_bytes((int)d.DL, (int)d.DR, (int)d.S, sizeof(T));
+    if(need > 200 * 1024) return HEFF_BAD_SHAPE;
     if(nb < 0) nb = d.cR;
     if(nb > 65535) return HEFF_BAD_SHAPE;
-    if(nb == 0) return HEFF_OK;
-    dim3 grid((unsigned)cdiv(d.cL, MIX_THREADS), (unsigned)nb);
-    HEFF_CUDA((launch_chained(mix_kernel<T>, grid, MIX_THREADS, smem, s, T1, T2, W, (int)d.S, (int)d.cL, (int)d.cR, (int)d.DL, (int)d.DR, (int)b0)));
-    return HEFF_OK;
+    MixArgs a{};
+    a.in = T1, a.out = T2, a.W = W;
+    a.K = (int)d.DL, a.J = (int)d.DR, a.S = (int)d.S, a.P = (int)d.cL, a.Q = (int)d.cR, a.q0 = (int)b0, a.nq = (int)nb;
+    a.in_k = d.cL, a.in_s = d.cL * d.DL, a.in_q = d.cL * d.DL * d.S;
+    a.w_k = 1, a.w_j = (int)d.DL, a.w_s = (int)(d.DL * d.DR), a.w_so = (int)(d.DL * d.DR * d.S);
+    return mpo_mix<CPLX>(a, s);
 }
 
 template<bool CPLX>

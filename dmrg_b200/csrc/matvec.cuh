@@ -46,6 +46,22 @@ struct MatvecScratch {
     }
 };
 
+// MPO mix at every point (p, q), p < P, q0 <= q < q0 + nq (< Q):
+//   out[s' + S (p + P (q + Q j))] = sum_{k,s} W[w_k k + w_j j + w_s s + w_so s'] in[p + in_q q + in_k k + in_s s],   j < J, k < K, s, s' < S
+struct MixArgs {
+    const void *in;
+    void       *out;
+    const void *W;
+    int         K, J, S, P, Q, q0, nq;
+    int64_t     in_k, in_s, in_q;
+    int         w_k, w_j, w_s, w_so;
+    bool        s_fastest;  // order of the sum: s fastest, or k
+    int         bufs;       // set by the launcher: tiles in flight,
+    bool        pairs, vec; // 16-byte stores of two s', 16-byte loads of two p (real)
+};
+template<bool CPLX>
+int mpo_mix(MixArgs a, cudaStream_t s);
+
 // Host-side address of the matvec's input permutation kernel (its first parameter is the input vector): a captured
 // matvec graph is retargeted to a new input through it.
 const void *permute_kernel_fn(bool cplx);
