@@ -325,14 +325,19 @@ int permute_R(const typename Scalar<CPLX>::T *R, typename Scalar<CPLX>::T *Rp, c
     return HEFF_OK;
 }
 
+// limit on the MPO's size: W, its nonzero list and 128 points of T1 within 200 KB
+template<bool CPLX>
+static bool mpo_too_large(const MatvecDims &d) {
+    const size_t es = CPLX ? 16 : 8;
+    return es * ((size_t)d.DL * d.DR * d.S * d.S + (size_t)d.DL * d.S * 128) + wlist_bytes((int)d.DL, (int)d.DR, (int)d.S, es) > 200 * 1024;
+}
+
 // T2[(s' + S a') + S cL (b + cR n)] = sum_{m,s} W[m + DL(n + DR(s + S s'))] T1[(a' + cL m) + cL DL (s + S b)], b0 <= b < b0 + nb
 template<bool CPLX>
 static int launch_mix(const MatvecDims &d, const typename Scalar<CPLX>::T *T1, typename Scalar<CPLX>::T *T2, const typename Scalar<CPLX>::T *W,
                       cudaStream_t s, int64_t b0 = 0, int64_t nb = -1) {
     using T = typename Scalar<CPLX>::T;
-    // limit on the MPO's size
-    const size_t need = sizeof(T) * ((size_t)d.DL * d.DR * d.S * d.S + (size_t)d.DL * d.S * 128) + wlist_bytes((int)d.DL, (int)d.DR, (int)d.S, sizeof(T));
-    if(need > 200 * 1024) return HEFF_BAD_SHAPE;
+    if(mpo_too_large<CPLX>(d)) return HEFF_BAD_SHAPE;
     if(nb < 0) nb = d.cR;
     if(nb > 65535) return HEFF_BAD_SHAPE;
     MixArgs a{};
@@ -348,6 +353,10 @@ int matvec_fp64(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename
                 const typename Scalar<CPLX>::T *Rp, const typename Scalar<CPLX>::T *W, const MatvecScratch<CPLX> &ws, cudaStream_t s,
                 cudaEvent_t *ev) {
     const int64_t n = d.size_mps();
+    if(!ev && matvec_fused_fits<CPLX>(d)) {
+        if(mpo_too_large<CPLX>(d)) return HEFF_BAD_SHAPE;
+        return matvec_fused<CPLX>(d, x, y, L, Rp, d.cR, d.cR * d.DR, W, s);
+    }
     if(ev) HEFF_CUDA(cudaEventRecord(ev[0], s));
     HEFF_CUDA((launch_chained(permute_mps_kernel<typename Scalar<CPLX>::T>, grid_1d(n), 256, 0, s, x, ws.xp, d.S, d.cL, n)));
     count_launches(2);  // the permutation and the MPO mix below (the GEMM launcher counts its own kernels)
@@ -595,6 +604,11 @@ static int matvec_stateless(void *res, const void *mps, const int64_t md[3], con
     if(res == mps) {
         set_last_error_msg("matvec: res must not alias mps");
         return HEFF_BAD_ARG;
+    }
+    if(matvec_fused_fits<CPLX>(d)) {  // R in the caller's layout
+        if(mpo_too_large<CPLX>(d)) return HEFF_BAD_SHAPE;
+        return matvec_fused<CPLX>(d, reinterpret_cast<const T *>(mps), reinterpret_cast<T *>(res), reinterpret_cast<const T *>(envL),
+                                  reinterpret_cast<const T *>(envR), d.cR * d.cR, d.cR, reinterpret_cast<const T *>(mpo), s);
     }
     const int64_t elems = MatvecScratch<CPLX>::elems(d) + MatvecScratch<CPLX>::pad(d.size_Rp());
     const size_t  split = matvec_split_bytes((size_t)elems * sizeof(T));

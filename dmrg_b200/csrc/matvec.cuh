@@ -4,7 +4,7 @@
 // 2*S*D*chiL*chiR*(chiL+chiR) + 2*S^2*DL*DR*chiL*chiR FLOPs, so one order serves both branches):
 //   P   x'[a,(s,b)]         = theta[s,a,b]                                    (layout, O(S chi^2))
 //   G1  T1[(a',m),(s,b)]    = sum_a  L[a,(a',m)] x'[a,(s,b)]                   (DMMA GEMM, K = chiL)
-//   MIX T2[(s',a'),(b,n)]   = sum_{m,s} W[m,n,s,s'] T1[(a',m),(s,b)]           (CUDA cores, per (a',b))
+//   MIX T2[(s',a'),(b,n)]   = sum_{m,s} W[m,n,s,s'] T1[(a',m),(s,b)]           (DMMA, per (a',b))
 //   G2  y[(s',a'),b']       = sum_{(b,n)} T2[(s',a'),(b,n)] R'[(b,n),b']       (DMMA GEMM, K = chiR*DR)
 // with R'[(b,n),b'] = R[b,b',n] permuted once per operator.  y lands directly in the
 // reference layout y[s' + S*(a' + chiL*b')].
@@ -89,7 +89,15 @@ int permute_mps(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename
 template<bool CPLX>
 int mix_fp64(const MatvecDims &d, const typename Scalar<CPLX>::T *T1, typename Scalar<CPLX>::T *T2, const typename Scalar<CPLX>::T *W, cudaStream_t s);
 
-// y = H_eff x with pre-permuted R'.  L and W in reference layout.  Launches 4 kernels on s.
+// The whole product in one launch (matvec_fused.cu), where matvec_fused_fits says that it is the faster way.  R element (b, b', n)
+// at R[b + r_bp b' + r_n n].
+template<bool CPLX>
+bool matvec_fused_fits(const MatvecDims &d);
+template<bool CPLX>
+int matvec_fused(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename Scalar<CPLX>::T *y, const typename Scalar<CPLX>::T *L,
+                 const typename Scalar<CPLX>::T *R, int64_t r_n, int64_t r_bp, const typename Scalar<CPLX>::T *W, cudaStream_t s);
+
+// y = H_eff x with pre-permuted R'.  L and W in reference layout.  Launches one fused kernel or four on s (always four with ev).
 // ev (optional): 5 events recorded before P and after P, G1, MIX, G2 (stage timing).
 template<bool CPLX>
 int matvec_fp64(const MatvecDims &d, const typename Scalar<CPLX>::T *x, typename Scalar<CPLX>::T *y, const typename Scalar<CPLX>::T *L,

@@ -627,7 +627,7 @@ static int apply_impl(heff_op *op, const void *x, void *y) {
         op->num_mv++;
         return HEFF_OK;
     }
-    if(op->graphs && !op->profiling && op->stream) {
+    if(op->graphs && !op->profiling && op->stream && !matvec_fused_fits<CPLX>(op->d)) {  // a single launch gains nothing from a graph
         if(op->mg && op->mg->matches(op, CPLX)) {
             HEFF_TRY(graph_replay<CPLX>(op, x, y));
         } else {
