@@ -488,6 +488,185 @@ static int orth_fast(const double2 *V, int64_t ldu, int64_t nu, int k, const dou
     return HEFF_OK;
 }
 
+// ---- orth_cgs2 in one launch for k <= 24 and vectors of at most ORTH_ONE_ROWS rows: one cluster does both passes of
+// orth_fast_kernel's modes, with the sums over the cluster pushed through distributed shared memory instead of partials in global
+// memory and a last block.  At these sizes the three launches wait for latencies: a launch, the loads of a row, the reduction's
+// tree, the atomic and the re-read of the partials, each time.  Every CTA adds the cluster's partial sums in rank order, so all of
+// them take the same decision on the second pass.  Eight CTAs where they hold the vector at one row per thread (the thread then
+// keeps its row of V in registers), else sixteen, whose threads re-read their rows from cache.  With the second pass taken, us,
+// three launches / one: k = 24 real n = 1024 20.6 / 7.2, 4096 21.0 / 7.2, 9216 20.7 / 12.5, 32768 23.0 / 18.5, complex 1024
+// 24.9 / 8.4, 8192 25.5 / 16.6; k = 7 real 4096 12.2 / 5.1.  Beyond, the bandwidth of sixteen SMs is the bound (complex k = 24
+// 16384 27.5 / 23.6).
+constexpr int64_t ORTH_ONE_ROWS = 16384;
+template<int P>
+__device__ __forceinline__ double orth_transpose_sum(double (&v)[P], int lane) {  // lane l: the warp's sum of column l mod P
+#pragma unroll
+    for(int off = P / 2; off > 0; off >>= 1)
+#pragma unroll
+        for(int j = 0; j < off; j++) {
+            const double send = (lane & off) ? v[j] : v[j + off];
+            v[j]              = ((lane & off) ? v[j + off] : v[j]) + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+#pragma unroll
+    for(int off = P; off < 32; off <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    return v[0];
+}
+
+constexpr int ORTH_ONE_THR = 256;
+template<bool CPLX, int KM, bool ONE>
+__global__ void __launch_bounds__(ORTH_ONE_THR, 1) orth_one_kernel(const double2 *V, int64_t ldu, int nu, int k, const double2 *in, double2 *out,
+                                                                   typename Scalar<CPLX>::T *__restrict__ hres) {
+    grid_wait();
+    constexpr int P = KM == 24 ? 32 : KM, WARPS = ORTH_ONE_THR / 32, CL = 16;  // at most 16 CTAs
+    __shared__ __align__(16) double2 sw[WARPS][P + 1];    // warp sums: columns, ||r||^2 in slot KM
+    __shared__ __align__(16) double2 sp[2][CL][KM + 1];   // partial sums of the cluster's CTAs, per pass
+    __shared__ double2               sh[2][KM + 1];
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x, cl = gridDim.x, step = cl * ORTH_ONE_THR;
+    const int i0 = rank * ORTH_ONE_THR + tid;
+    double2   v[KM], r = make_double2(0.0, 0.0);
+    double    are[P], aim[CPLX ? P : 1], nrm = 0.0;
+    auto      load = [&](int i) {
+#pragma unroll
+        for(int j = 0; j < KM; j++) v[j] = i < nu ? V[i + ldu * (j < k ? j : 0)] : make_double2(0.0, 0.0);
+    };
+    auto clear = [&]() {
+        nrm = 0.0;
+#pragma unroll
+        for(int j = 0; j < P; j++) {
+            are[j] = 0.0;
+            if constexpr(CPLX) aim[j] = 0.0;
+        }
+    };
+    auto dots = [&]() {
+#pragma unroll
+        for(int j = 0; j < KM; j++)
+            if(j < k) {
+                are[j] = fma(v[j].x, r.x, fma(v[j].y, r.y, are[j]));  // complex: conj(v) r
+                if constexpr(CPLX) aim[j] = fma(v[j].x, r.y, fma(-v[j].y, r.x, aim[j]));
+            }
+        nrm = fma(r.x, r.x, fma(r.y, r.y, nrm));
+    };
+    auto project = [&](const double2 *h, double scale) {
+        double ax = 0, ay = 0;
+#pragma unroll
+        for(int j = 0; j < KM; j++)
+            if(j < k) {
+                if constexpr(CPLX) {
+                    ax = fma(v[j].x, h[j].x, fma(-v[j].y, h[j].y, ax));
+                    ay = fma(v[j].x, h[j].y, fma(v[j].y, h[j].x, ay));
+                } else {
+                    ax = fma(v[j].x, h[j].x, ax);
+                    ay = fma(v[j].y, h[j].x, ay);
+                }
+            }
+        r = make_double2((r.x - ax) * scale, (r.y - ay) * scale);
+    };
+    // sums over the cluster into sh[pass]; returns sum |h_j|^2
+    auto reduce = [&](int pass) {
+        if constexpr(KM == 24) are[KM] = nrm;
+        const double sre = orth_transpose_sum<P>(are, lane);
+        double       sim = 0.0;
+        if constexpr(CPLX) sim = orth_transpose_sum<P>(aim, lane);
+        if(lane < P) sw[warp][lane] = make_double2(sre, sim);
+        if constexpr(KM != 24) {
+#pragma unroll
+            for(int off = 16; off > 0; off >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, off);
+            if(lane == 0) sw[warp][KM] = make_double2(nrm, 0.0);
+        }
+        __syncthreads();
+        if(pass == 0) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // every CTA has started
+        for(int e = tid; e < (k + 1) * cl; e += ORTH_ONE_THR) {
+            const int j = e / cl, src = j < k ? j : KM;
+            double    a = 0, b = 0;
+#pragma unroll
+            for(int w = 0; w < WARPS; w++) a += sw[w][src].x, b += sw[w][src].y;
+            uint32_t addr;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(&sp[pass][rank][src])), "r"(e % cl));
+            asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};\n" ::"r"(addr), "d"(a), "d"(b) : "memory");
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        if(tid <= k) {
+            const int src = tid < k ? tid : KM;
+            double    a = 0, b = 0;
+            for(int q = 0; q < cl; q++) a += sp[pass][q][src].x, b += sp[pass][q][src].y;
+            sh[pass][src] = make_double2(a, CPLX ? b : 0.0);
+        }
+        __syncthreads();
+        double h2 = 0.0;
+        if(lane < k) h2 = sh[pass][lane].x * sh[pass][lane].x + sh[pass][lane].y * sh[pass][lane].y;
+#pragma unroll
+        for(int off = 16; off > 0; off >>= 1) h2 += __shfl_xor_sync(0xffffffffu, h2, off);
+        return h2;
+    };
+    clear();
+#pragma unroll 1
+    for(int i = i0; i < (ONE ? i0 + 1 : nu); i += step) {
+        load(i);
+        r = i < nu ? in[i] : make_double2(0.0, 0.0);
+        dots();
+    }
+    const double hn1 = reduce(0), w2 = sh[0][KM].x;
+    double       beta2  = w2 - hn1;
+    const bool   second = !(beta2 > 0.5 * w2);  // severe cancellation: orthogonalise again
+    const double s1     = second ? 1.0 : (beta2 > 1e-300 ? 1.0 / sqrt(beta2) : 0.0);
+    clear();
+#pragma unroll 1
+    for(int i = i0; i < (ONE ? i0 + 1 : nu); i += step) {
+        if(!ONE) {
+            load(i);
+            r = in[i];
+        }
+        project(sh[0], s1);
+        if(second) dots();
+        if((!ONE || !second) && i < nu) out[i] = r;
+    }
+    if(second) {  // uniform over the cluster
+        const double hn2 = reduce(1), v2 = sh[1][KM].x;
+        beta2            = v2 - hn2;
+        const double s2  = beta2 > 1e-300 ? 1.0 / sqrt(beta2) : 0.0;
+#pragma unroll 1
+        for(int i = i0; i < (ONE ? i0 + 1 : nu); i += step) {
+            if(!ONE) {
+                load(i);
+                r = out[i];
+            }
+            project(sh[1], s2);
+            if(i < nu) out[i] = r;
+        }
+    }
+    if(rank == 0) {
+        using T = typename Scalar<CPLX>::T;
+        if(tid < k) {
+            double2 h = sh[0][tid];
+            if(second) h = make_double2(h.x + sh[1][tid].x, h.y + sh[1][tid].y);
+            hres[tid] = orth_make<T>(h.x, h.y);
+        }
+        if(tid == 0) {
+            hres[k]     = orth_make<T>(sqrt(fmax(beta2, 0.0)), 0.0);
+            hres[k + 1] = orth_make<T>(w2, second ? 1.0 : 0.0);
+        }
+    }
+}
+
+template<bool CPLX, int KM>
+static int orth_one(const double2 *V, int64_t ldu, int64_t nu, int k, const double2 *w, double2 *v, typename Scalar<CPLX>::T *hres, cudaStream_t s) {
+    if(nu <= 8 * ORTH_ONE_THR) {
+        HEFF_CUDA((launch_chained_cluster(8u, orth_one_kernel<CPLX, KM, true>, dim3(8), dim3(ORTH_ONE_THR), 0, s, V, ldu, (int)nu, k, w, v, hres)));
+        return HEFF_OK;
+    }
+    static int attr_done[64] = {0};
+    int        dev           = 0;
+    HEFF_CUDA(cudaGetDevice(&dev));
+    if(dev < 0 || dev >= 64 || !attr_done[dev]) {
+        HEFF_CUDA(cudaFuncSetAttribute(orth_one_kernel<CPLX, KM, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        if(dev >= 0 && dev < 64) attr_done[dev] = 1;
+    }
+    HEFF_CUDA((launch_chained_cluster(16u, orth_one_kernel<CPLX, KM, false>, dim3(16), dim3(ORTH_ONE_THR), 0, s, V, ldu, (int)nu, k, w, v, hres)));
+    return HEFF_OK;
+}
+
 template<bool CPLX>
 int orth_cgs2(const typename Scalar<CPLX>::T *V, int64_t ldv, int64_t n, int k, const typename Scalar<CPLX>::T *w, typename Scalar<CPLX>::T *v,
               double *partials, unsigned *counter, double *st, typename Scalar<CPLX>::T *hres, cudaStream_t s) {
@@ -500,6 +679,11 @@ int orth_cgs2(const typename Scalar<CPLX>::T *V, int64_t ldv, int64_t n, int k, 
         const int64_t  ldu = CPLX ? ldv : ldv / 2, nu = CPLX ? n : n / 2;
         const double2 *w2  = reinterpret_cast<const double2 *>(w);
         double2       *v2  = reinterpret_cast<double2 *>(v);
+        if(nu <= ORTH_ONE_ROWS) {
+            if(k <= 8) return orth_one<CPLX, 8>(V2, ldu, nu, k, w2, v2, hres, s);
+            if(k <= 16) return orth_one<CPLX, 16>(V2, ldu, nu, k, w2, v2, hres, s);
+            return orth_one<CPLX, 24>(V2, ldu, nu, k, w2, v2, hres, s);
+        }
         if(k <= 8) return orth_fast<CPLX, 8>(V2, ldu, nu, k, w2, v2, partials, counter, st, hres, s);
         if(k <= 16) return orth_fast<CPLX, 16>(V2, ldu, nu, k, w2, v2, partials, counter, st, hres, s);
         return orth_fast<CPLX, 24>(V2, ldu, nu, k, w2, v2, partials, counter, st, hres, s);

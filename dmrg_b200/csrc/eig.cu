@@ -116,7 +116,7 @@ struct Davidson {
     int                    maxb, minb;
     T *V = nullptr, *AV = nullptr, *V2 = nullptr, *AV2 = nullptr, *t = nullptr, *x = nullptr, *ax = nullptr, *r = nullptr;
     T *cg_p = nullptr, *cg_q = nullptr, *cg_z = nullptr, *cg_d = nullptr, *cg_r = nullptr;
-    T *dh = nullptr, *dc = nullptr, *hres = nullptr;
+    T *dh = nullptr, *dc = nullptr;
     double             *partials = nullptr, *dscal = nullptr, *orth_st = nullptr, *cg_cs = nullptr;
     unsigned           *orth_counter = nullptr;
     std::vector<HT>     Hk, G2;
@@ -178,7 +178,6 @@ struct Davidson {
         HEFF_TRY(take((void **)&dc, es * MD_MAXK * MD_MAXK));
         HEFF_TRY(take((void **)&partials, sizeof(double) * MD_BLOCKS * MD_MAXK * 4));
         HEFF_TRY(take((void **)&dscal, sizeof(double) * 16));
-        HEFF_TRY(take((void **)&hres, es * (MD_MAXK + 2)));
         HEFF_TRY(take((void **)&orth_st, sizeof(double) * (8 + 4 * (MD_MAXK + 2))));
         HEFF_TRY(take((void **)&orth_counter, 256));
         HEFF_TRY(take((void **)&cg_cs, sizeof(double) * 16));
@@ -376,8 +375,7 @@ struct Davidson {
         double              best = INFINITY, verify = 1.0;
         while(true) {
             T *vk = V + (int64_t)k * n;  // slot of the next basis vector
-            HEFF_TRY(orth_cgs2<CPLX>(V, n, n, k, AV + (int64_t)(k - 1) * n, vk, partials, orth_counter, orth_st, hres, s));
-            HEFF_CUDA(cudaMemcpyAsync(hh, hres, sizeof(T) * (k + 2), cudaMemcpyDeviceToHost, s));
+            HEFF_TRY(orth_cgs2<CPLX>(V, n, n, k, AV + (int64_t)(k - 1) * n, vk, partials, orth_counter, orth_st, hh, s));  // the coefficients land in pinned memory
             HEFF_CUDA(cudaEventRecord(op->eig_event, s));
             // the product of v_k, needed by the next iteration unless the solve stops here
             HEFF_TRY(apply(vk, AV + (int64_t)k * n, !use_mixed));
