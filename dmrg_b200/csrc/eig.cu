@@ -89,18 +89,19 @@ static std::vector<int> ritz_order(const std::vector<double> &w, int rule, doubl
     return o;
 }
 
-// Pinned host buffer and event through which the Krylov loop reads each iteration's coefficients while
-// the next matvec runs (created once per operator).
+// Pinned host buffers and events through which the Krylov loop reads each iteration's coefficients while
+// the next matvec runs (two of each, created once per operator).
 int eig_host_ready(heff_op *op) {
     if(!op->eig_host) {
-        cudaError_t e = cudaMallocHost(&op->eig_host, sizeof(double2) * (MD_MAXK + 2));
+        cudaError_t e = cudaMallocHost(&op->eig_host, 2 * sizeof(double2) * (MD_MAXK + 2));
         if(e != cudaSuccess) {
             op->eig_host = nullptr;
             set_last_cuda_error(e, "eigensolver host buffer", __FILE__, __LINE__);
             return HEFF_OOM;
         }
     }
-    if(!op->eig_event) HEFF_CUDA(cudaEventCreateWithFlags(&op->eig_event, cudaEventDisableTiming));
+    for(cudaEvent_t &e : op->eig_event)
+        if(!e) HEFF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return HEFF_OK;
 }
 
@@ -352,12 +353,52 @@ struct Davidson {
         return scale(V, 1.0 / std::sqrt(n2));
     }
 
+    // Step k on the stream: v_k from A v_{k-1}, its coefficients to the pinned slot hh, ev after them.
+    int expand(int k, T *hh, cudaEvent_t ev) {
+        HEFF_TRY(orth_cgs2<CPLX>(V, n, n, k, AV + (int64_t)(k - 1) * n, V + (int64_t)k * n, partials, orth_counter, orth_st, hh, s));
+        HEFF_CUDA(cudaEventRecord(ev, s));
+        return HEFF_OK;
+    }
+    // Selected Ritz value, the modulus of its vector's last component, and the largest |Ritz value| of the k x k problem.
+    int ritz_values(int k, double &theta, double &last, double &amax) {
+        std::vector<HT> &a = small_a;
+        a.resize((size_t)k * k);
+        for(int j = 0; j < k; j++)
+            for(int i = 0; i < k; i++) a[i + (size_t)k * j] = 0.5 * (Hk[i + (size_t)maxb * j] + HostScalar<CPLX>::conj(Hk[j + (size_t)maxb * i]));
+        std::vector<double> &w = small_w, &z = small_z;
+        if(last_row_eig(k, a, w, z)) {  // its plain QL gave up: the full decomposition scales each step
+            std::vector<HT> v;
+            HEFF_TRY(ritz<CPLX>(k, Hk, maxb, w, v));
+            z.resize(k);
+            for(int i = 0; i < k; i++) z[i] = std::abs(v[k - 1 + (size_t)k * i]);
+        }
+        int b = 0;
+        for(int i = 1; i < k; i++) {
+            const bool better = cfg.ritz == HEFF_RITZ_LA      ? w[i] > w[b]
+                                : cfg.ritz == HEFF_RITZ_TARGET ? std::fabs(w[i] - cfg.target) < std::fabs(w[b] - cfg.target)
+                                                               : w[i] < w[b];
+            if(better) b = i;
+        }
+        theta = w[b];
+        last  = z[b];
+        for(double wi : w) amax = std::max(amax, std::fabs(wi));
+        return HEFF_OK;
+    }
+    std::vector<HT>     small_a;
+    std::vector<double> small_w, small_z;
+
+    // Vectors up to this length (elements): the next expansion step is queued behind the product before the host reads the
+    // current one's coefficients, so the stream never waits for the host's Rayleigh-Ritz step; the one that a stop leaves unused
+    // writes only the free basis column and its own slot.  Longer products hide the host by themselves.
+    static constexpr int64_t AHEAD_MAX = 1 << 18;
+
     // Phase 1 (thick-restart Krylov / Lanczos structure).  With w = A v_{k-1} projected out of V_k,
     //   A V_k = V_k H_k + beta v_k e_k^H,
     // so the projection coefficients ARE the last column of the Rayleigh-Ritz matrix H_k and the Ritz
     // residual norm is |beta * s_{k-1}|.  The projection (with its DGKS second pass) and the normalisation of
-    // v_k run on the device (orth_cgs2), so the product A v_k is enqueued before the host reads the
-    // coefficients: the host's Rayleigh-Ritz step overlaps the GPU's matvec.  A thick restart keeps
+    // v_k run on the device (orth_cgs2), so the product A v_k (and for short vectors the next step, AHEAD_MAX) is
+    // enqueued before the host reads the coefficients: the host's Rayleigh-Ritz step, which asks for the selected
+    // value and its vector's last component only until the solve stops or restarts, overlaps the GPU's work.  A thick restart keeps
     // Y = V_k S_m (all residuals along v_k) and appends v_k with its product, preserving the relation.
     // Returns x = Ritz vector (normalised), theta, rnorm (explicit when converged).
     int run(const void *x0, bool use_mixed, double stop_tol, int64_t max_mv, double &theta, double &rnorm, bool &conv) {
@@ -370,16 +411,22 @@ struct Davidson {
         int                 k = 1;
         std::vector<double> w;
         std::vector<HT>     vecs;
-        T                  *hh    = reinterpret_cast<T *>(op->eig_host);
+        T                  *slot[2] = {reinterpret_cast<T *>(op->eig_host), reinterpret_cast<T *>(op->eig_host) + MD_MAXK + 2};
+        int                 cur     = 0;  // slot of the step that the host waits for
+        bool                queued  = false;  // that step is on the stream already
+        const bool          ahead   = n <= AHEAD_MAX;
         int                 stagn = 0;
         double              best = INFINITY, verify = 1.0;
         while(true) {
-            T *vk = V + (int64_t)k * n;  // slot of the next basis vector
-            HEFF_TRY(orth_cgs2<CPLX>(V, n, n, k, AV + (int64_t)(k - 1) * n, vk, partials, orth_counter, orth_st, hh, s));  // the coefficients land in pinned memory
-            HEFF_CUDA(cudaEventRecord(op->eig_event, s));
+            T *vk = V + (int64_t)k * n;  // the next basis vector
+            if(!queued) HEFF_TRY(expand(k, slot[cur], op->eig_event[cur]));
             // the product of v_k, needed by the next iteration unless the solve stops here
             HEFF_TRY(apply(vk, AV + (int64_t)k * n, !use_mixed));
-            HEFF_CUDA(cudaEventSynchronize(op->eig_event));
+            queued = ahead && k < maxb;
+            if(queued) HEFF_TRY(expand(k + 1, slot[cur ^ 1], op->eig_event[cur ^ 1]));
+            HEFF_CUDA(cudaEventSynchronize(op->eig_event[cur]));
+            const T *hh = slot[cur];
+            cur ^= 1;
             std::vector<HT> h(k, HT(0));
             for(int i = 0; i < k; i++) std::memcpy((void *)&h[i], (void *)&hh[i], sizeof(T));
             HT bt, wf;
@@ -394,15 +441,26 @@ struct Davidson {
                 Hk[i + (size_t)maxb * (k - 1)] = h[i];
                 Hk[(k - 1) + (size_t)maxb * i] = HostScalar<CPLX>::conj(h[i]);
             }
-            HEFF_TRY(ritz<CPLX>(k, Hk, maxb, w, vecs));
-            for(double wi : w) anorm = std::max(anorm, std::fabs(wi));
-            const std::vector<int> ord = ritz_order(w, cfg.ritz, cfg.target);
-            theta                      = w[ord[0]];
-            const HT *sv               = vecs.data() + (size_t)k * ord[0];
-            const double est           = beta * std::abs(std::complex<double>(sv[k - 1]));
-            rnorm                      = est;
+            double last = 0.0, amax = 0.0;  // of the selected Ritz pair: its vector's last component; largest |Ritz value|
+            HEFF_TRY(ritz_values(k, theta, last, amax));
+            anorm            = std::max(anorm, amax);
+            const double est = beta * last;
+            rnorm            = est;
             res.iters++;
+            // the Ritz vectors, where the iteration stops or restarts
+            std::vector<int> ord;
+            const HT        *sv   = nullptr;
+            auto             full = [&]() -> int {
+                if(sv) return HEFF_OK;
+                HEFF_TRY(ritz<CPLX>(k, Hk, maxb, w, vecs));
+                for(double wi : w) anorm = std::max(anorm, std::fabs(wi));
+                ord   = ritz_order(w, cfg.ritz, cfg.target);
+                theta = w[ord[0]];
+                sv    = vecs.data() + (size_t)k * ord[0];
+                return HEFF_OK;
+            };
             if(est <= verify * stop_tol * std::max(anorm, 1e-300) || res.num_mv >= max_mv) {
+                HEFF_TRY(full());
                 HEFF_TRY(explicit_residual(k, sv, theta, rnorm));
                 if(!std::isfinite(rnorm)) {
                     set_last_error_msg("eigensolver: non-finite residual");
@@ -420,18 +478,21 @@ struct Davidson {
                     best  = est;
                     stagn = 0;
                 } else if(++stagn >= 20) {
+                    HEFF_TRY(full());
                     HEFF_TRY(explicit_residual(k, sv, theta, rnorm));
                     break;
                 }
             }
             if(!(beta > 1e-13 * std::sqrt(std::max(w2, 1e-300)))) {
                 // invariant subspace: the Ritz pair is exact for this operator
+                HEFF_TRY(full());
                 HEFF_TRY(explicit_residual(k, sv, theta, rnorm));
                 conv = rnorm <= stop_tol * std::max(anorm, 1e-300);
                 break;
             }
             if(k == maxb) {
                 // keep minb Ritz vectors, then append v_k and its product
+                HEFF_TRY(full());
                 HEFF_TRY(restart(k, minb, w, vecs, ord, false));  // swaps V <-> V2, AV <-> AV2: v_k is now V2[:, k]
                 HEFF_CUDA(cudaMemcpyAsync(V + (int64_t)minb * n, V2 + (int64_t)k * n, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
                 HEFF_CUDA(cudaMemcpyAsync(AV + (int64_t)minb * n, AV2 + (int64_t)k * n, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));

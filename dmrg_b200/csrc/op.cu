@@ -690,7 +690,8 @@ extern "C" int heff_op_destroy(heff_op *op) {
     if(op->diag) cudaFree(op->diag);
     if(op->jcb) cudaFree(op->jcb);
     if(op->eig_host) cudaFreeHost(op->eig_host);
-    if(op->eig_event) cudaEventDestroy(op->eig_event);
+    for(cudaEvent_t e : op->eig_event)
+        if(e) cudaEventDestroy(e);
     delete op;
     return HEFF_OK;
 }

@@ -44,7 +44,7 @@ struct heff_op {
     void              *eig_ws       = nullptr;
     size_t             eig_ws_bytes = 0;
     void              *eig_host     = nullptr;  // pinned: per-iteration coefficients (Krylov loop)
-    cudaEvent_t        eig_event    = nullptr;
+    cudaEvent_t        eig_event[2] = {};
     // diagonal of H_eff for the Jacobi preconditioner (computed on first use after create / rebind)
     void              *diag         = nullptr;
     int64_t            diag_cap     = 0;

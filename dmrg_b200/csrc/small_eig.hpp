@@ -16,6 +16,7 @@
 #include <cmath>
 #include <complex>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 namespace heff {
@@ -182,6 +183,109 @@ inline int herm_eig(int k, const std::vector<std::complex<double>> &h, std::vect
         w.push_back(ww[c]);
     }
     return (int)w.size() == k ? 0 : 1;
+}
+
+// Eigenvalues of a Hermitian matrix (ascending order not implied) and the modulus of each eigenvector's LAST component, which is
+// all that a Krylov iteration asks of its Rayleigh-Ritz problem until it stops or restarts.  The Householder reduction takes the
+// rows from the last one up, so its transformations leave the last basis vector alone, and the QL rotations are applied to the
+// last row of the eigenvector matrix only; a complex matrix is reduced as it is (phases of the off-diagonals change neither the
+// eigenvalues nor the moduli) instead of through the real form of twice the order.  us for k = 24: all eigenvectors real 45,
+// complex 280; this real 25, complex 43.  a: n x n, column-major, overwritten.
+template<class T>
+inline int last_row_eig(int n, std::vector<T> &a, std::vector<double> &d, std::vector<double> &z) {
+    auto cj  = [](const T &v) { if constexpr(std::is_same_v<T, double>) return v; else return std::conj(v); };
+    auto ab2 = [](const T &v) { if constexpr(std::is_same_v<T, double>) return v * v; else return std::norm(v); };
+    auto re  = [](const T &v) { if constexpr(std::is_same_v<T, double>) return v; else return v.real(); };
+    d.assign(n, 0.0);
+    z.assign(n, 0.0);
+    if(n == 0) return 0;
+    double big = 0.0;
+    for(const T &v : a) big = std::max(big, std::max(std::fabs(re(v)), std::abs(v)));
+    if(!std::isfinite(big)) return 1;
+    int ex = 0;
+    if(big > 0.0) std::frexp(big, &ex);  // scaled to below one, so squares neither overflow nor lose anything that matters
+    const double down = std::ldexp(1.0, -ex / 2), down2 = std::ldexp(1.0, -ex - (-ex / 2));
+    for(T &v : a) v = v * down * down2;
+    std::vector<double> e(n, 0.0);
+    std::vector<T>      u(n), q(n);
+    for(int i = n - 1; i > 0; i--) {
+        T           *c = a.data() + (size_t)n * i;  // column i, rows 0 .. i - 1
+        const int    l = i - 1;
+        double       off = 0.0;
+        for(int k = 0; k < l; k++) off += ab2(c[k]);
+        const double cl2 = ab2(c[l]), nrm = std::sqrt(off + cl2);
+        e[i] = nrm;
+        d[i] = re(c[i]);
+        if(off == 0.0) continue;
+        const double cl = std::sqrt(cl2);
+        const T      ph = cl > 0.0 ? T(c[l] / cl) : T(1.0);
+        for(int k = 0; k < l; k++) u[k] = c[k];
+        u[l] = c[l] + ph * nrm;  // (I - beta u u^H) c = -ph |c| e_l
+        const double beta = 1.0 / (nrm * (nrm + cl));
+        for(int k = 0; k < i; k++) q[k] = T(0.0);
+        for(int j = 0; j < i; j++) {
+            const T *col = a.data() + (size_t)n * j;
+            const T  uj  = u[j] * beta;
+            for(int k = 0; k < i; k++) q[k] += col[k] * uj;
+        }
+        double h = 0.0;
+        for(int k = 0; k < i; k++) h += re(cj(u[k]) * q[k]);
+        h *= 0.5 * beta;
+        for(int k = 0; k < i; k++) q[k] -= h * u[k];
+        for(int j = 0; j < i; j++) {
+            T      *col = a.data() + (size_t)n * j;
+            const T qj = cj(q[j]), uj = cj(u[j]);
+            for(int k = 0; k < i; k++) col[k] -= u[k] * qj + q[k] * uj;
+        }
+    }
+    d[0]     = re(a[0]);
+    z[n - 1] = 1.0;
+    for(int i = 1; i < n; i++) e[i - 1] = e[i];
+    e[n - 1] = 0.0;
+    for(int l = 0; l < n; l++) {  // implicit QL, as in sym_eig
+        for(int iter = 0;; iter++) {
+            int m = l;
+            for(; m < n - 1; m++)
+                if(std::fabs(e[m]) <= 1e-300 || std::fabs(e[m]) <= 2.2e-16 * (std::fabs(d[m]) + std::fabs(d[m + 1]))) break;
+            if(m == l) break;
+            if(iter == 60) return 1;
+            double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+            double r = std::hypot(g, 1.0);
+            g        = d[m] - d[l] + e[l] / (g + (g >= 0 ? r : -r));
+            double s = 1.0, c = 1.0, p = 0.0;
+            int    i = m - 1;
+            for(; i >= l; i--) {
+                const double f = s * e[i], b = c * e[i];
+                r        = std::sqrt(f * f + g * g);
+                e[i + 1] = r;
+                if(r == 0.0) {
+                    d[i + 1] -= p;
+                    e[m] = 0.0;
+                    break;
+                }
+                const double ir = 1.0 / r;
+                s        = f * ir;
+                c        = g * ir;
+                g        = d[i + 1] - p;
+                r        = (d[i] - g) * s + 2.0 * c * b;
+                p        = s * r;
+                d[i + 1] = g + p;
+                g        = c * r - b;
+                const double zi = z[i], zj = z[i + 1];
+                z[i + 1] = s * zi + c * zj;
+                z[i]     = c * zi - s * zj;
+            }
+            if(r == 0.0 && i >= l) continue;
+            d[l] -= p;
+            e[l] = g;
+            e[m] = 0.0;
+        }
+    }
+    for(int i = 0; i < n; i++) {
+        d[i] = std::ldexp(d[i], ex);
+        z[i] = std::fabs(z[i]);
+    }
+    return 0;
 }
 
 }  // namespace heff
