@@ -50,7 +50,7 @@ __device__ __forceinline__ void x_store(const XGemmArgs &p, int row, int n, floa
 // Persistent CTA (one per SM): walks the tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (grouped order)
 //   warp 0 lane 0: TMA producer over the k-blocks of all its tiles (one continuous smem ring)
 //   warp 1 lane 0: MMA issuer into TMEM accumulator buffer (j & 1) for the CTA's j-th tile
-//   warps 2-5:     epilogue of tile j from buffer (j & 1) while the MMAs of tile j+1 run in the other buffer
+//   other warps:   epilogue of tile j from buffer (j & 1) while the MMAs of tile j+1 run in the other buffer
 __global__ void __launch_bounds__(X_THREADS, 1)
     gemm_bf16x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const XGemmArgs p) {
     grid_wait();
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(X_THREADS, 1)
         }
         for(int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 128);
+            mbar_init(&acc_empty[b], X_EPI);
         }
         *s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(X_THREADS, 1)
             }
         }
     } else {
-        // epilogue: warps 2..5 -> TMEM lane quarters 2,3,0,1
-        const int q = warp & 3;
+        // epilogue: warp -> TMEM lane quarter warp & 3, column group (warp - 2) / 4
+        constexpr int CW = X_BN * 128 / X_EPI;
+        const int     q = warp & 3, c0 = ((warp - 2) >> 2) * CW;
         int       j = 0;
         for(int t = blockIdx.x; t < ntiles; t += gridDim.x, j++) {
             const int buf = j & 1;
@@ -151,11 +152,11 @@ __global__ void __launch_bounds__(X_THREADS, 1)
                 atomicExch(p.err, 3);
                 atomicOr(s_fail, 1);
             }
-            epi_bar();  // every epilogue warp takes the same decision
+            epi_bar<X_EPI>();  // every epilogue warp takes the same decision
             if(*s_fail) break;
             fence_after();
             const int row = m0 + q * 32 + lane;
-            for(int c = 0; c < X_BN; c += 32) {
+            for(int c = c0; c < c0 + CW; c += 32) {
                 uint32_t r[32];
                 tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * X_BN + c), r);
                 if(row < p.M) {
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(X_THREADS, 1)
             }
             fence_before();
             mbar_arrive(&acc_empty[buf]);  // TMEM buffer free for the tile after next
-            epi_bar();                     // *s_fail is read by all before the next wait may set it
+            epi_bar<X_EPI>();                     // *s_fail is read by all before the next wait may set it
         }
     }
     fence_before();

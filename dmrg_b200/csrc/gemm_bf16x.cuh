@@ -19,7 +19,7 @@
 
 namespace heff {
 
-constexpr int X_BM = 128, X_BN = 256, X_BK = 64, X_STAGES = 4, X_THREADS = 192;
+constexpr int X_BM = 128, X_BN = 256, X_BK = 64, X_STAGES = 4, X_EPI = 512, X_THREADS = 64 + X_EPI;
 constexpr int X_A_BYTES     = X_BM * X_BK * 2;  // 16 KB
 constexpr int X_B_BYTES     = X_BN * X_BK * 2;  // 32 KB
 constexpr int X_STAGE_BYTES = X_A_BYTES + X_B_BYTES;

@@ -97,8 +97,9 @@ __device__ __forceinline__ void z_digits16(double (&y)[16], uint32_t (&w)[4], ui
         w[q] = 0u, wn[q] = 0u;
 #pragma unroll
         for(int j = 0; j < 4; j++) {
-            const int d = __double2int_rn(y[4 * q + j]);
-            y[4 * q + j] = (y[4 * q + j] - (double)d) * 128.0;
+            const double t = y[4 * q + j] + 6755399441055744.0;  // 1.5 * 2^52: rint in the low word, no conversion instruction
+            const int    d = __double2loint(t);
+            y[4 * q + j] = (y[4 * q + j] - (t - 6755399441055744.0)) * 128.0;
             w[q] |= ((uint32_t)d & 0xffu) << (8 * j);
             wn[q] |= ((uint32_t)(-d) & 0xffu) << (8 * j);
         }
@@ -288,75 +289,86 @@ __device__ __forceinline__ void z_tile_mn(const ZGemmArgs &p, int tile, int &m0,
     n0                  = ((tile % per_group) / gsize) * BN;
 }
 
-// Level g of tile (m0, n0) from TMEM columns [col0, col0 + BN) into C: the first level processed (g = s-1)
-// stores, the others add.  All loads of a 32-column chunk are issued before its stores.
+// INT32 -> FP64 by a magic number, exact: an integer and an FP64 instruction, at twice the rate of the conversion (29 and 15 per
+// clock and SM).
+__device__ __forceinline__ double z_i2d(uint32_t r) { return __hiloint2double(0x43300000, (int)(r ^ 0x80000000u)) - 4503601774854144.0; }
+__device__ __forceinline__ double z_level(int g) { return __hiloint2double((1023 - 7 * g) << 20, 0); }  // 2^-7g
 __device__ __forceinline__ double z_nan() { return __longlong_as_double(0x7ff8000000000000ll); }
 
-template<int BN>
-__device__ __forceinline__ void z_epilogue(const ZGemmArgs &p, uint32_t tmem_row, int row, int n0, int g, bool poison) {
-    const bool first = g == p.nslice - 1;
-    double     lv    = 1.0;
-    for(int i = 0; i < g; i++) lv *= 0.0078125;  // 2^-7g, exact
-    const double ra = row < p.M ? (poison ? z_nan() : p.fa[row] * lv) : 0.0;
-    for(int c = 0; c < BN; c += 32) {
-        uint32_t r[32];
-        tmem_ld32(tmem_row + (uint32_t)c, r);
+// Column factors of a tile in shared memory (zero beyond N), by the epilogue threads before the tile's first level.
+template<int BN, int EPI>
+__device__ __forceinline__ void z_factors(const ZGemmArgs &p, double *sfb, int n0) {
+    for(int i = (int)threadIdx.x - 64; i < BN; i += EPI) sfb[i] = n0 + i < p.N ? p.fb[p.cplx ? (n0 + i) >> 1 : n0 + i] : 0.0;
+}
+
+// 16 columns from n1 of one row: C (+)= r * (ra f).  FULL chunks (all columns below N) run without a test or a branch per column:
+// the tests had made the epilogue, not the MMAs, the bound of short levels.
+template<bool CPLX, bool FULL>
+__device__ __forceinline__ void z_add16(const ZGemmArgs &p, const uint32_t (&r)[16], const double *sf, int row, int n1, double ra, bool first) {
+    if constexpr(!CPLX) {
+        double *C = reinterpret_cast<double *>(p.C) + row + p.ldc * n1;
+        double  old[16];
+#pragma unroll
+        for(int jj = 0; jj < 16; jj++) old[jj] = 0.0;
+        if(!first) {
+#pragma unroll
+            for(int jj = 0; jj < 16; jj++)
+                if(FULL || n1 + jj < p.N) old[jj] = C[p.ldc * jj];
+        }
+#pragma unroll
+        for(int jj = 0; jj < 16; jj++)
+            if(FULL || n1 + jj < p.N) C[p.ldc * jj] = old[jj] + z_i2d(r[jj]) * (ra * sf[jj]);  // the product is exact
+    } else {
+        double2 *C = reinterpret_cast<double2 *>(p.C) + row + p.ldc * (n1 >> 1);
+        double2  old[8];
+#pragma unroll
+        for(int jj = 0; jj < 8; jj++) old[jj] = make_double2(0.0, 0.0);
+        if(!first) {
+#pragma unroll
+            for(int jj = 0; jj < 8; jj++)
+                if(FULL || n1 + 2 * jj < p.N) old[jj] = C[p.ldc * jj];
+        }
+#pragma unroll
+        for(int jj = 0; jj < 8; jj++)
+            if(FULL || n1 + 2 * jj < p.N) {  // N is even
+                const double s = ra * sf[2 * jj];
+                C[p.ldc * jj] = make_double2(old[jj].x + z_i2d(r[2 * jj]) * s, old[jj].y + z_i2d(r[2 * jj + 1]) * s);
+            }
+    }
+}
+
+// Level g of columns [c0, c1) of tile (m0, n0) from TMEM into C: the first level processed (g = s-1) stores, the others add.
+__device__ __forceinline__ void z_epilogue(const ZGemmArgs &p, uint32_t tmem_row, const double *sfb, int row, int n0, int g, bool poison, int c0, int c1) {
+    const bool   first = g == p.nslice - 1;
+    const double ra    = row < p.M ? (poison ? z_nan() : p.fa[row] * z_level(g)) : 0.0;
+#pragma unroll 1
+    for(int c = c0; c < c1; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(tmem_row + (uint32_t)c, r);
         if(row >= p.M) continue;
+        const int n1 = n0 + c;
         if(!p.cplx) {
-            double *C = reinterpret_cast<double *>(p.C) + row;
-#pragma unroll
-            for(int h = 0; h < 32; h += 16) {
-                double old[16], f[16];
-#pragma unroll
-                for(int jj = 0; jj < 16; jj++) {
-                    const int n = n0 + c + h + jj;
-                    f[jj] = old[jj] = 0.0;
-                    if(n < p.N) {
-                        f[jj] = __ldg(p.fb + n);
-                        if(!first) old[jj] = C[p.ldc * n];
-                    }
-                }
-#pragma unroll
-                for(int jj = 0; jj < 16; jj++) {
-                    const int n = n0 + c + h + jj;
-                    if(n < p.N) C[p.ldc * n] = old[jj] + (double)(int)r[h + jj] * (ra * f[jj]);  // the product is exact
-                }
-            }
+            if(n1 + 16 <= p.N)
+                z_add16<false, true>(p, r, sfb + c, row, n1, ra, first);
+            else
+                z_add16<false, false>(p, r, sfb + c, row, n1, ra, first);
         } else {
-            double2 *C = reinterpret_cast<double2 *>(p.C) + row;
-            double2  old[16];
-            double   f[16];
-#pragma unroll
-            for(int jj = 0; jj < 16; jj++) {
-                const int n = n0 + c + 2 * jj;  // even; n + 1 < N whenever n < N
-                f[jj] = 0.0, old[jj] = make_double2(0.0, 0.0);
-                if(n < p.N) {
-                    f[jj] = __ldg(p.fb + (n >> 1));
-                    if(!first) old[jj] = C[p.ldc * (n >> 1)];
-                }
-            }
-#pragma unroll
-            for(int jj = 0; jj < 16; jj++) {
-                const int n = n0 + c + 2 * jj;
-                if(n < p.N) {
-                    const double s = ra * f[jj];
-                    C[p.ldc * (n >> 1)] = make_double2(old[jj].x + (double)(int)r[2 * jj] * s, old[jj].y + (double)(int)r[2 * jj + 1] * s);
-                }
-            }
+            if(n1 + 16 <= p.N)
+                z_add16<true, true>(p, r, sfb + c, row, n1, ra, first);
+            else
+                z_add16<true, false>(p, r, sfb + c, row, n1, ra, first);
         }
     }
 }
 
-// Level g of tile (m0, n0) with the FP64 sum over levels kept in TMEM (TMEM_SUM tiles): INT32 accumulator at
-// tacc, FP64 partial at tpart (column pairs lo, hi); the same FP64 operations in the same order as z_epilogue,
-// so both give identical results.  The last level (g = 0) writes C once.
-template<int BN>
-__device__ __forceinline__ void z_epilogue_tsum(const ZGemmArgs &p, uint32_t tacc, uint32_t tpart, int row, int n0, int g, bool poison) {
-    const bool first = g == p.nslice - 1, last = g == 0;
-    double     lv    = 1.0;
-    for(int i = 0; i < g; i++) lv *= 0.0078125;  // 2^-7g, exact
-    const double ra = row < p.M ? (poison ? z_nan() : p.fa[row] * lv) : 0.0;
-    for(int c = 0; c < BN; c += 32) {
+// The same with the FP64 sum over levels kept in TMEM (TMEM_SUM tiles): INT32 accumulator at tacc, FP64 partial at tpart (column
+// pairs lo, hi); the same FP64 operations in the same order as z_epilogue, so both give identical results.  The last level (g = 0)
+// writes C once.
+__device__ __forceinline__ void z_epilogue_tsum(const ZGemmArgs &p, uint32_t tacc, uint32_t tpart, const double *sfb, int row, int n0, int g, bool poison,
+                                                int c0, int c1) {
+    const bool   first = g == p.nslice - 1, last = g == 0;
+    const double ra    = row < p.M ? (poison ? z_nan() : p.fa[row] * z_level(g)) : 0.0;
+    for(int c = c0; c < c1; c += 32) {
         uint32_t r[32];
         tmem_ld32(tacc + (uint32_t)c, r);
 #pragma unroll
@@ -366,11 +378,8 @@ __device__ __forceinline__ void z_epilogue_tsum(const ZGemmArgs &p, uint32_t tac
             if(!first) tmem_ld32(tpart + (uint32_t)(2 * (c + h)), w);
 #pragma unroll
             for(int jj = 0; jj < 16; jj++) {
-                const int    n  = n0 + c + h + jj;
-                const int    nb = p.cplx ? (n >> 1) : n;
-                const double f  = n < p.N ? __ldg(p.fb + nb) : 0.0;
-                const double x  = (double)(int)r[h + jj] * (ra * f);  // exact
-                v[jj]           = first ? x : __hiloint2double((int)w[2 * jj + 1], (int)w[2 * jj]) + x;
+                const double x = z_i2d(r[h + jj]) * (ra * sfb[c + h + jj]);  // exact
+                v[jj]          = first ? x : __hiloint2double((int)w[2 * jj + 1], (int)w[2 * jj]) + x;
             }
             if(!last) {
 #pragma unroll
@@ -401,13 +410,13 @@ __device__ __forceinline__ void z_epilogue_tsum(const ZGemmArgs &p, uint32_t tac
     if(!last) tmem_wait_st();
 }
 
-// Persistent CTA (one per SM) over units (tile t, level g), t = blockIdx.x, blockIdx.x + gridDim.x, ...,
+// Persistent CTA (one per SM, tiles of 128 x 128 or 192) over units (tile t, level g), t = blockIdx.x, blockIdx.x + gridDim.x, ...,
 // g = s-1 .. 0; unit j of the CTA accumulates in TMEM buffer (j & 1).
 //   warp 0 lane 0: TMA producer: unit (t, g) streams k-blocks of slice pairs (i, g - i), i = 0..g
 //   warp 1 lane 0: MMA issuer
-//   warps 2-5:     epilogue of unit j while the MMAs of unit j+1 run in the other buffer
+//   other warps:   epilogue of unit j while the MMAs of unit j+1 run in the other buffer
 template<int BN>
-__global__ void __launch_bounds__(Z_THREADS, 1)
+__global__ void __launch_bounds__(ZCfg<BN>::THREADS, 1)
     gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ZGemmArgs p) {
     grid_wait();
     extern __shared__ __align__(1024) unsigned char zsm_raw[];
@@ -419,6 +428,7 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
     uint64_t      *acc_empty = acc_full + 2;      // [2]
     uint32_t      *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
     int           *s_fail    = reinterpret_cast<int *>(tmem_slot + 1);
+    double        *sfb       = reinterpret_cast<double *>(smem + Cfg::STAGES * Cfg::STAGE + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntiles = ((p.M + Z_BM - 1) / Z_BM) * ((p.N + BN - 1) / BN);
@@ -432,7 +442,7 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
         }
         for(int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 128);
+            mbar_init(&acc_empty[b], Cfg::EPI);
         }
         *s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -507,8 +517,9 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
             }
         }
     } else {
-        // epilogue: warps 2..5 -> TMEM lane quarters 2,3,0,1
-        const int  q      = warp & 3;
+        // epilogue: warp -> TMEM lane quarter warp & 3, column group (warp - 2) / 4
+        constexpr int CW = BN * 128 / Cfg::EPI;
+        const int  q = warp & 3, c0 = ((warp - 2) >> 2) * CW;
         int        j      = 0;
         bool       stop   = false;
         const bool poison = (*p.bad_a | *p.bad_b) != 0;  // raised by the slicers, which ran before this kernel
@@ -516,13 +527,14 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
         for(int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
             int m0, n0;
             z_tile_mn<BN>(p, t, m0, n0);
+            z_factors<BN, Cfg::EPI>(p, sfb, n0);  // the barrier after the wait orders it before its use, the one below after its last
             for(int g = ns - 1; g >= 0; g--, j++) {
                 const int buf = j & 1;
                 if(!mbar_wait(&acc_full[buf], (j >> 1) & 1)) {
                     atomicExch(p.err, 3);
                     atomicOr(s_fail, 1);
                 }
-                epi_bar();  // every epilogue warp takes the same decision
+                epi_bar<Cfg::EPI>();  // every epilogue warp takes the same decision
                 if(*s_fail) {
                     stop = true;
                     break;
@@ -530,12 +542,12 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
                 fence_after();
                 const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16);
                 if constexpr(ZCfg<BN>::TMEM_SUM)
-                    z_epilogue_tsum<BN>(p, trow + (uint32_t)(buf * BN), trow + (uint32_t)ZCfg<BN>::PART_COL, m0 + q * 32 + lane, n0, g, poison);
+                    z_epilogue_tsum(p, trow + (uint32_t)(buf * BN), trow + (uint32_t)ZCfg<BN>::PART_COL, sfb, m0 + q * 32 + lane, n0, g, poison, c0, c0 + CW);
                 else
-                    z_epilogue<BN>(p, trow + (uint32_t)(buf * BN), m0 + q * 32 + lane, n0, g, poison);
+                    z_epilogue(p, trow + (uint32_t)(buf * BN), sfb, m0 + q * 32 + lane, n0, g, poison, c0, c0 + CW);
                 fence_before();
                 mbar_arrive(&acc_empty[buf]);  // TMEM buffer free for the unit after next
-                epi_bar();                     // *s_fail is read by all before the next wait may set it
+                epi_bar<Cfg::EPI>();                     // *s_fail is read by all before the next wait may set it
             }
         }
     }
@@ -544,6 +556,172 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
     if(warp == 1) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::TMEM_COLS) : "memory");
+    }
+}
+
+// CTA pair on a tile of 256 x 256 (tcgen05 cta_group::2): each CTA holds 128 rows of A and 128 of the tile's 256 rows of B, so a
+// k-block brings 32 KB into an SM for the same 128 x 256 x 128 products that a lone CTA needs 48 KB for, and what an SM can take
+// in (about 54 B/clk) bounds the main loop: the products of a real chi = 1000 matvec without their epilogue take 398 and 247 us by
+// lone CTAs and 290 and 211 by pairs (181 at the pipe's rate).  With it 599 and 335 before, 435 and 293 now: the levels summed in
+// C share that intake.
+// Same roles as above; the even CTA's warp 1 issues the MMAs of both.  Its full barriers count both CTAs' bytes and its acc_empty
+// both CTAs' epilogue threads; commits arrive in both CTAs.
+constexpr uint32_t Z_IDESC_PAIR = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(2 * Z_BM >> 4) << 24);
+__device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(Z_IDESC_PAIR), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void z_pair_mn(const ZGemmArgs &p, int tile, int &m0, int &n0) {
+    const int num_m = (p.M + 2 * Z_BM - 1) / (2 * Z_BM), num_n = (p.N + 255) / 256, group = Z_GROUP_M / 2;
+    const int per_group = group * num_n, first_m = (tile / per_group) * group, gsize = min(num_m - first_m, group);
+    m0 = (first_m + (tile % per_group) % gsize) * 2 * Z_BM;
+    n0 = ((tile % per_group) / gsize) * 256;
+}
+__global__ void __launch_bounds__(ZPair::THREADS, 1)
+    gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ZGemmArgs p) {
+    grid_wait();
+    extern __shared__ __align__(1024) unsigned char zsm_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(zsm_raw) + 1023) & ~uintptr_t(1023));
+    using Cfg            = ZPair;
+    uint64_t *full       = reinterpret_cast<uint64_t *>(smem + Cfg::STAGES * Cfg::STAGE);
+    uint64_t *empty      = full + Cfg::STAGES;
+    uint64_t *acc_full   = empty + Cfg::STAGES;  // [2]
+    uint64_t *acc_empty  = acc_full + 2;         // [2]
+    uint32_t *tmem_slot  = reinterpret_cast<uint32_t *>(acc_empty + 2);
+    int      *s_fail     = reinterpret_cast<int *>(tmem_slot + 1);
+    double   *sfb        = reinterpret_cast<double *>(smem + Cfg::STAGES * Cfg::STAGE + 256);
+
+    const int  warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)pair_rank();
+    const int  ntiles = ((p.M + 2 * Z_BM - 1) / (2 * Z_BM)) * ((p.N + 255) / 256);
+    const int  KBs = (p.K + Z_BK - 1) / Z_BK, ns = p.nslice;  // k-blocks per slice
+    const int  t0 = (int)blockIdx.x >> 1, tstep = (int)gridDim.x >> 1;
+
+    if(threadIdx.x == 0) {
+        for(int s = 0; s < Cfg::STAGES; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for(int b = 0; b < 2; b++) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 2 * Cfg::EPI);
+        }
+        *s_fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if(warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    pair_sync();  // both CTAs' barriers and TMEM are ready
+    fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if(warp == 0) {
+        if(lane == 0) {  // TMA producer of this CTA's halves
+            int  it = 0;
+            bool ok = true;
+            for(int t = t0; t < ntiles && ok; t += tstep) {
+                int m0, n0;
+                z_pair_mn(p, t, m0, n0);
+                for(int g = ns - 1; g >= 0 && ok; g--) {
+                    const int nkb = (g + 1) * KBs;
+                    for(int kb = 0; kb < nkb; kb++, it++) {
+                        const int      st = it % Cfg::STAGES;
+                        const uint32_t ph = (it / Cfg::STAGES) & 1;
+                        if(!mbar_wait(&empty[st], ph ^ 1)) {
+                            atomicExch(p.err, 1);
+                            ok = false;
+                            break;
+                        }
+                        const int      i  = kb / KBs;  // A slice i, B slice g - i
+                        const int      k0 = (kb - i * KBs) * Z_BK;
+                        unsigned char *a = smem + st * Cfg::STAGE, *b = a + Z_A_BYTES;
+                        if(rank == 0) mbar_expect_tx(&full[st], 2 * Cfg::STAGE);
+                        const uint32_t bar = leader_addr(&full[st]);
+                        tma_load_3d_pair(&tmA, bar, a, k0, m0 + rank * Z_BM, i);
+                        tma_load_3d_pair(&tmB, bar, b, k0, n0 + rank * 128, g - i);
+                    }
+                }
+            }
+        }
+    } else if(warp == 1) {
+        if(lane == 0 && rank == 0) {  // MMA issuer of the pair
+            int  it = 0, j = 0;
+            bool ok = true;
+            for(int t = t0; t < ntiles && ok; t += tstep) {
+                for(int g = ns - 1; g >= 0 && ok; g--, j++) {
+                    const int      buf = j & 1;
+                    const uint32_t acc = tmem_base + (uint32_t)(buf * 256);
+                    if(!mbar_wait(&acc_empty[buf], ((j >> 1) & 1) ^ 1)) {  // both epilogues drained this buffer
+                        atomicExch(p.err, 4);
+                        ok = false;
+                        break;
+                    }
+                    fence_after();
+                    const int nkb = (g + 1) * KBs;
+                    for(int kb = 0; kb < nkb; kb++, it++) {
+                        const int      st = it % Cfg::STAGES;
+                        const uint32_t ph = (it / Cfg::STAGES) & 1;
+                        if(!mbar_wait(&full[st], ph)) {
+                            atomicExch(p.err, 2);
+                            ok = false;
+                            break;
+                        }
+                        fence_after();
+                        const uint32_t a = saddr(smem + st * Cfg::STAGE), b = a + Z_A_BYTES;
+#pragma unroll
+                        for(int k = 0; k < Z_BK / 32; k++) umma_i8_pair(acc, sdesc_sw128(a + 32 * k), sdesc_sw128(b + 32 * k), (kb | k) != 0);
+                        umma_commit_pair(&empty[st]);
+                    }
+                    if(ok) umma_commit_pair(&acc_full[buf]);  // fires when every MMA of this unit has completed
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // epilogue of this CTA's 128 rows
+        constexpr int CW = 256 * 128 / Cfg::EPI;
+        const int  q = warp & 3, c0 = ((warp - 2) >> 2) * CW;
+        int        j      = 0;
+        bool       stop   = false;
+        const bool poison = (*p.bad_a | *p.bad_b) != 0;  // raised by the slicers, which ran before this kernel
+        if(poison && threadIdx.x == 64) atomicExch(p.err, 5);
+        for(int t = t0; t < ntiles && !stop; t += tstep) {
+            int m0, n0;
+            z_pair_mn(p, t, m0, n0);
+            z_factors<256, Cfg::EPI>(p, sfb, n0);
+            for(int g = ns - 1; g >= 0; g--, j++) {
+                const int buf = j & 1;
+                if(!mbar_wait(&acc_full[buf], (j >> 1) & 1)) {
+                    atomicExch(p.err, 3);
+                    atomicOr(s_fail, 1);
+                }
+                epi_bar<Cfg::EPI>();  // every epilogue warp takes the same decision
+                if(*s_fail) {
+                    stop = true;
+                    break;
+                }
+                fence_after();
+                z_epilogue(p, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256), sfb, m0 + rank * Z_BM + q * 32 + lane, n0, g, poison, c0, c0 + CW);
+                fence_before();
+                mbar_arrive_cluster(leader_addr(&acc_empty[buf]));  // TMEM buffer free for the unit after next
+                epi_bar<Cfg::EPI>();                                          // *s_fail is read by all before the next wait may set it
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    pair_sync();  // the pair's MMAs and remote arrivals are done
+    if(warp == 1) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
 }
 
@@ -600,17 +778,17 @@ static int z_forced_bn() {
 
 int z_choose_bn(int64_t M, int64_t N, int64_t K) {
     if(const int forced = z_forced_bn(); forced >= 128) return forced;
-    // cost = waves x width x per-MAC weight.  The weights are measured (B200, 7 slices, the matvec GEMMs of
-    // chi=1024, real and complex): with few k-blocks per slice the levels are short and summing them in C
-    // costs more than the 128-wide tile's extra operand traffic; with long K the widest tile is best.
+    // cost = waves x width x per-MAC weight (the 256-wide tile is a CTA pair's, two rows of tiles at once).  The weights are
+    // measured (7 slices, the real matvec GEMMs of chi = 1000, us at 256 / 192 / 128: K = 1000 435 / 535 / 533, K = 3000
+    // 293 / 520 / 535): the pair moves the least operand data, and the 128-wide tile's level sum in TMEM pays for short K only.
     const int64_t sms  = device_sm_count();
     const int64_t kbs  = cdiv(K, Z_BK);
     const int     bn[3] = {256, 192, 128};
-    const double  w[3]  = {1.0, kbs <= 16 ? 0.95 : 1.06, kbs <= 8 ? 0.85 : 1.3};
+    const double  w[3]  = {1.0, 1.2, kbs <= 8 ? 1.2 : 1.8};
     int           best = 256;
     double        bc   = 1e300;
     for(int i = 0; i < 3; i++) {
-        const int64_t tiles = cdiv(M, Z_BM) * cdiv(N, bn[i]);
+        const int64_t tiles = (bn[i] == 256 ? 2 * cdiv(M, 2 * Z_BM) : cdiv(M, Z_BM)) * cdiv(N, bn[i]);
         const double  c     = (double)cdiv(tiles, sms) * bn[i] * w[i];
         if(c < bc * 0.999) bc = c, best = bn[i];
     }
@@ -629,15 +807,30 @@ static int z_launch(const CUtensorMap &tA, const CUtensorMap &tB, const ZGemmArg
     const int64_t tiles = cdiv(a.M, Z_BM) * cdiv(a.N, BN);
     if(tiles > 0x7fffffff) return HEFF_BAD_SHAPE;
     const int grid = (int)std::min<int64_t>(tiles, device_sm_count());
-    HEFF_CUDA((launch_chained(gemm_i8_kernel<BN>, (unsigned)grid, Z_THREADS, ZCfg<BN>::SMEM, s, tA, tB, a)));
+    HEFF_CUDA((launch_chained(gemm_i8_kernel<BN>, (unsigned)grid, ZCfg<BN>::THREADS, ZCfg<BN>::SMEM, s, tA, tB, a)));
+    return HEFF_OK;
+}
+
+static int z_launch_pair(const CUtensorMap &tA, const CUtensorMap &tB, const ZGemmArgs &a, cudaStream_t s) {
+    static int attr_done[64] = {0};
+    int        dev           = 0;
+    HEFF_CUDA(cudaGetDevice(&dev));
+    if(dev < 0 || dev >= 64 || !attr_done[dev]) {
+        HEFF_CUDA(cudaFuncSetAttribute(gemm_i8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ZPair::SMEM));
+        if(dev >= 0 && dev < 64) attr_done[dev] = 1;
+    }
+    const int64_t tiles = cdiv(a.M, 2 * Z_BM) * cdiv(a.N, 256);
+    if(tiles > 0x3fffffff) return HEFF_BAD_SHAPE;
+    const int grid = 2 * (int)std::min<int64_t>(tiles, std::max(1, device_sm_count() / 2));
+    HEFF_CUDA((launch_chained_cluster(2u, gemm_i8_pair_kernel, dim3((unsigned)grid), dim3(ZPair::THREADS), (size_t)ZPair::SMEM, s, tA, tB, a)));
     return HEFF_OK;
 }
 
 static int z_launch_bn(int bn, const ZPlanes &A, const ZPlanes &B, const ZGemmArgs &a, cudaStream_t s) {
     CUtensorMap tA, tB;
     HEFF_TRY(make_tmap_planes(&tA, A, Z_BM));
-    HEFF_TRY(make_tmap_planes(&tB, B, bn));
-    if(bn == 256) return z_launch<256>(tA, tB, a, s);
+    HEFF_TRY(make_tmap_planes(&tB, B, bn == 256 ? 128 : bn));  // at 256 a CTA of the pair loads half of B
+    if(bn == 256) return z_launch_pair(tA, tB, a, s);
     if(bn == 192) return z_launch<192>(tA, tB, a, s);
     return z_launch<128>(tA, tB, a, s);
 }

@@ -20,9 +20,9 @@
 // Complex operands use a real embedding: A' rows [re | im], B' rows 2n = [re | -im] and 2n+1 = [im | re],
 // so C'[m, 2n] = Re C[m, n] and C'[m, 2n+1] = Im C[m, n] with one real GEMM of K' = 2K.
 //
-// CTA: 192 threads = warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer, warps 2-5 epilogue.  Tile
-// 128 x BN (BN = 128, 192 or 256), k-block 128 bytes, 4-6-stage ring, two TMEM accumulators; persistent (one
-// CTA per SM) over the (tile, level) units.  Every mbarrier wait is bounded; on timeout *err is raised, the
+// CTA: 320 threads = warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer, warps 2-9 epilogue.  Tile
+// 128 x BN (BN = 128 or 192) of a CTA or 256 x 256 of a CTA pair, k-block 128 bytes, 5-6-stage ring, two TMEM
+// accumulators; persistent (one CTA per SM) over the (tile, level) units.  Every mbarrier wait is bounded; on timeout *err is raised, the
 // CTA skips its remaining work, frees its TMEM and returns.  No cluster multicast.
 #pragma once
 #include <cuda.h>
@@ -31,20 +31,26 @@
 
 namespace heff {
 
-constexpr int Z_BM = 128, Z_BK = 128, Z_THREADS = 192;
+constexpr int Z_BM = 128, Z_BK = 128;
 constexpr int Z_A_BYTES = Z_BM * Z_BK;  // 16 KB
-// Tile width BN in {128, 192, 256} (chosen per shape to fill the last wave): the ring takes as many stages of
-// A (16 KB) + B (BN x 128 B) as fit in 210 KB.  At BN = 128 the FP64 sum over levels stays in TMEM (two INT32
+// Tile width in {128, 192, 256} (chosen per shape), 256 by CTA pairs (ZPair).  The ring of a lone CTA takes as many
+// stages of A (16 KB) + B (BN x 128 B) as fit in 210 KB.  At BN = 128 the FP64 sum over levels stays in TMEM (two INT32
 // accumulators in columns [0, 256), the FP64 partial as b32 pairs in [256, 512)) and C is written once; at the
 // wider tiles TMEM holds only the two accumulators and the levels are summed in C (L2-resident).
+// EPI epilogue threads: four warps per group of BN * 128 / EPI columns.
 template<int BN>
 struct ZCfg {
+    static constexpr int  EPI        = 256, THREADS = 64 + EPI;
     static constexpr int  STAGE      = Z_A_BYTES + BN * Z_BK;
-    static constexpr int  STAGES     = (210 * 1024) / STAGE;  // 4, 5, 6
-    static constexpr int  SMEM       = STAGES * STAGE + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int  STAGES     = (210 * 1024) / STAGE;  // 6, 5
+    static constexpr int  SMEM       = STAGES * STAGE + 1024 /*align*/ + 256 /*barriers*/ + 8 * BN /*column factors*/;
     static constexpr bool TMEM_SUM   = BN == 128;
     static constexpr int  TMEM_COLS  = 512;
     static constexpr int  PART_COL   = 2 * BN;  // first column of the FP64 partial (TMEM_SUM)
+};
+struct ZPair {  // 256 x 256 tiles by CTA pairs
+    static constexpr int EPI = 256, THREADS = 64 + EPI;
+    static constexpr int STAGE = Z_A_BYTES + 128 * Z_BK, STAGES = 6, SMEM = STAGES * STAGE + 1024 + 256 + 8 * 256;
 };
 constexpr int Z_MAX_SLICES  = 8;
 constexpr int Z_DEFAULT_SLICES = 7;
