@@ -71,8 +71,8 @@ struct EmuSizes {
 };
 static EmuSizes emu_sizes(const EmuDims &e, int ns, int64_t rmax_rows) {
     EmuSizes z;
-    z.A1 = up256((size_t)ns * e.M1 * e.kx1), z.B1 = up256((size_t)ns * e.cf * e.N1 * e.kx1);
-    z.A2 = up256((size_t)ns * e.M2 * e.kx2), z.B2 = up256((size_t)ns * e.cf * e.N2 * e.kx2);
+    z.A1 = up256((size_t)ns * e.M1 * z_ld(e.kx1)), z.B1 = up256((size_t)ns * e.cf * e.N1 * z_ld(e.kx1));
+    z.A2 = up256((size_t)ns * e.M2 * z_ld(e.kx2)), z.B2 = up256((size_t)ns * e.cf * e.N2 * z_ld(e.kx2));
     z.S  = up256(sizeof(double) * 2 * (size_t)(e.M1 + e.N1 + e.M2 + e.N2));
     z.R  = up256(sizeof(unsigned long long) * (size_t)rmax_rows);
     return z;
@@ -116,7 +116,7 @@ static int emu_layout(heff_op *op, EmuState *st) {
     st->B2.inv = sc, st->B2.fac = sc + e.N2;
     p += z.S;
     auto planes = [&](ZPlanes &q, size_t bytes, int64_t rows, int64_t kx) {
-        q.planes = reinterpret_cast<int8_t *>(p), q.rows = rows, q.kx = kx, q.nslice = ns;
+        q.planes = reinterpret_cast<int8_t *>(p), q.rows = rows, q.kx = kx, q.ld = z_ld(kx), q.nslice = ns;
         p += bytes;
     };
     planes(st->A1, z.A1, e.M1, e.kx1);

@@ -7,11 +7,11 @@
 // and the split products are folded into the K dimension (A' = [a_hi | a_hi | a_mid],
 // B' = [b_hi | b_mid | b_hi] gives a_hi b_hi + a_hi b_mid + a_mid b_hi in one GEMM).
 //
-// CTA: 192 threads = warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer, warps 2-5 epilogue
-// (tcgen05.ld 32x32b: warp w reads TMEM lanes 32*(w%4) .. +31).  Tile 128 x 256 x 64.  Persistent: one CTA
-// per SM walks its share of the tiles with two TMEM accumulators (512 columns), so the epilogue of a tile
-// overlaps the MMAs of the next.  Every mbarrier wait is bounded: on timeout the kernel raises *err, skips its
-// remaining work, still frees its TMEM and returns.  No cluster multicast anywhere.
+// CTA pairs (tcgen05 cta_group::2) on tiles of 256 x 256 x 64: each CTA holds 128 rows of A and 128 of B's.  A CTA has warp 0 TMA producer of its halves, warp 1 TMEM allocator and, in the even CTA, MMA issuer of the pair, the other
+// warps epilogue of its 128 rows (tcgen05.ld 32x32b: warp w reads TMEM lanes 32*(w%4) .. +31).  Persistent: the pairs walk their
+// share of the tiles with two TMEM accumulators, so the epilogue of a tile overlaps the MMAs of the next.  Every mbarrier wait is
+// bounded: on timeout the kernel raises *err, skips its remaining work, still frees its TMEM and returns.  No cluster multicast
+// of loads anywhere.
 #pragma once
 #include <cuda.h>
 
@@ -19,10 +19,10 @@
 
 namespace heff {
 
-constexpr int X_BM = 128, X_BN = 256, X_BK = 64, X_STAGES = 4, X_EPI = 512, X_THREADS = 64 + X_EPI;
-constexpr int X_A_BYTES     = X_BM * X_BK * 2;  // 16 KB
-constexpr int X_B_BYTES     = X_BN * X_BK * 2;  // 32 KB
-constexpr int X_STAGE_BYTES = X_A_BYTES + X_B_BYTES;
+constexpr int X_BM = 128, X_BN = 256, X_BK = 64, X_STAGES = 6, X_EPI = 512, X_THREADS = 64 + X_EPI;
+constexpr int X_A_BYTES     = X_BM * X_BK * 2;      // 16 KB
+constexpr int X_BOX_B       = X_BN / 2;             // rows of B in one CTA
+constexpr int X_STAGE_BYTES = X_A_BYTES + X_BOX_B * X_BK * 2;
 constexpr int X_SMEM_BYTES  = X_STAGES * X_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 
 enum XEpilogue : int {
@@ -44,7 +44,7 @@ struct XGemmArgs {
 // Builds a 2D K-major bf16 tensor map over rows x kcols (row pitch ld_elems) with box {64, box_rows}.
 int make_tmap_bf16(CUtensorMap *map, const void *base, int64_t rows, int64_t kcols, int64_t ld_elems, int box_rows);
 
-// Launch one BF16 GEMM.  tmA covers A (M x K, box rows 128), tmB covers B (N x K, box rows 256).
+// Launch one BF16 GEMM.  tmA covers A (M x K, box rows 128), tmB covers B (N x K, box rows X_BOX_B).
 int gemm_bf16x(const CUtensorMap &tmA, const CUtensorMap &tmB, const XGemmArgs &args, cudaStream_t s);
 
 }  // namespace heff

@@ -116,7 +116,7 @@ __device__ __forceinline__ bool z_bad16(const double (&y)[16]) {
 
 // Writes the ns digit planes of a 16-column group g of source row r (yr, yi already scaled by 64 / sigma_r).
 template<bool CPLX, bool BMODE>
-__device__ __forceinline__ void z_emit(double (&yr)[16], double (&yi)[16], int8_t *planes, int64_t plane, int64_t kx, int64_t Kh, int64_t r,
+__device__ __forceinline__ void z_emit(double (&yr)[16], double (&yi)[16], int8_t *planes, int64_t plane, int64_t pitch, int64_t Kh, int64_t r,
                                        int64_t g, int ns, int *bad) {
     if(z_bad16(yr) || (CPLX && z_bad16(yi))) atomicExch(bad, 1);
     for(int t = 0; t < ns; t++) {
@@ -124,17 +124,17 @@ __device__ __forceinline__ void z_emit(double (&yr)[16], double (&yi)[16], int8_
         z_digits16(yr, wr, wnr);
         int8_t *base = planes + t * plane;
         if constexpr(!CPLX) {
-            z_st16(base + r * kx + g * 16, wr);
+            z_st16(base + r * pitch + g * 16, wr);
         } else {
             z_digits16(yi, wi, wni);
             if constexpr(!BMODE) {  // [re | im]
-                z_st16(base + r * kx + g * 16, wr);
-                z_st16(base + r * kx + Kh + g * 16, wi);
+                z_st16(base + r * pitch + g * 16, wr);
+                z_st16(base + r * pitch + Kh + g * 16, wi);
             } else {  // 2r: [re | -im], 2r + 1: [im | re]
-                z_st16(base + (2 * r) * kx + g * 16, wr);
-                z_st16(base + (2 * r) * kx + Kh + g * 16, wni);
-                z_st16(base + (2 * r + 1) * kx + g * 16, wi);
-                z_st16(base + (2 * r + 1) * kx + Kh + g * 16, wr);
+                z_st16(base + (2 * r) * pitch + g * 16, wr);
+                z_st16(base + (2 * r) * pitch + Kh + g * 16, wni);
+                z_st16(base + (2 * r + 1) * pitch + g * 16, wi);
+                z_st16(base + (2 * r + 1) * pitch + Kh + g * 16, wr);
             }
         }
     }
@@ -143,10 +143,10 @@ __device__ __forceinline__ void z_emit(double (&yr)[16], double (&yi)[16], int8_
 // K-major source: thread per (row, 16-column group), groups of a row on consecutive threads
 template<bool CPLX, bool BMODE>
 __global__ void __launch_bounds__(256) z_slice_k_kernel(const typename Scalar<CPLX>::T *__restrict__ src, int64_t rows, int64_t K, int64_t ld,
-                                                         const double *__restrict__ inv, int8_t *__restrict__ planes, int64_t prow, int64_t kx, int ns,
+                                                         const double *__restrict__ inv, int8_t *__restrict__ planes, int64_t prow, int64_t pitch, int ns,
                                                          int *bad) {
     grid_wait();
-    const int64_t ng = (K + 15) / 16, Kh = ng * 16, tot = rows * ng, plane = prow * kx;
+    const int64_t ng = (K + 15) / 16, Kh = ng * 16, tot = rows * ng, plane = prow * pitch;
     for(int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t g = e % ng, r = e / ng;
         const double  sc = inv[r];
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256) z_slice_k_kernel(const typename Scalar<CP
                 yi[j]        = z_im(v) * sc;
             }
         }
-        z_emit<CPLX, BMODE>(yr, yi, planes, plane, kx, Kh, r, g, ns, bad);
+        z_emit<CPLX, BMODE>(yr, yi, planes, plane, pitch, Kh, r, g, ns, bad);
     }
 }
 
@@ -171,12 +171,12 @@ __global__ void __launch_bounds__(256) z_slice_k_kernel(const typename Scalar<CP
 constexpr int ZM_TR = 32, ZM_TK = 64, ZM_THREADS = ZM_TR * ZM_TK / 16;
 template<bool CPLX>
 __global__ void __launch_bounds__(ZM_THREADS) z_slice_m_kernel(const typename Scalar<CPLX>::T *__restrict__ src, int64_t rows, int64_t K,
-                                                                int64_t ld, const double *__restrict__ inv, int8_t *__restrict__ planes, int64_t kx,
+                                                                int64_t ld, const double *__restrict__ inv, int8_t *__restrict__ planes, int64_t pitch,
                                                                 int ns, int *bad) {
     grid_wait();
     using T = typename Scalar<CPLX>::T;
     __shared__ T  tile[ZM_TK][ZM_TR + 1];
-    const int64_t ng = (K + 15) / 16, Kh = ng * 16, plane = rows * kx;
+    const int64_t ng = (K + 15) / 16, Kh = ng * 16, plane = rows * pitch;
     const int64_t r0 = (int64_t)blockIdx.x * ZM_TR, k0 = (int64_t)blockIdx.y * ZM_TK;
     for(int idx = threadIdx.x; idx < ZM_TR * ZM_TK; idx += ZM_THREADS) {
         const int     rl = idx % ZM_TR, kl = idx / ZM_TR;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(ZM_THREADS) z_slice_m_kernel(const typename Sc
         yr[j]     = z_re(v) * sc;
         yi[j]     = z_im(v) * sc;
     }
-    z_emit<CPLX, false>(yr, yi, planes, plane, kx, Kh, r, g, ns, bad);
+    z_emit<CPLX, false>(yr, yi, planes, plane, pitch, Kh, r, g, ns, bad);
 }
 
 static int z_grid(int64_t n, int per_block = 256) {
@@ -233,9 +233,9 @@ int z_slice_kmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
     if(rows <= 0) return HEFF_OK;
     const int64_t tot = rows * cdiv(K, 16);
     if(CPLX && bmode)
-        HEFF_CUDA((launch_chained(z_slice_k_kernel<CPLX, true>, z_grid(tot), 256, 0, s, src, rows, K, ld, p.inv, p.planes, p.rows, p.kx, p.nslice, bad)));
+        HEFF_CUDA((launch_chained(z_slice_k_kernel<CPLX, true>, z_grid(tot), 256, 0, s, src, rows, K, ld, p.inv, p.planes, p.rows, p.ld, p.nslice, bad)));
     else
-        HEFF_CUDA((launch_chained(z_slice_k_kernel<CPLX, false>, z_grid(tot), 256, 0, s, src, rows, K, ld, p.inv, p.planes, p.rows, p.kx, p.nslice, bad)));
+        HEFF_CUDA((launch_chained(z_slice_k_kernel<CPLX, false>, z_grid(tot), 256, 0, s, src, rows, K, ld, p.inv, p.planes, p.rows, p.ld, p.nslice, bad)));
     return HEFF_OK;
 }
 
@@ -244,7 +244,7 @@ int z_slice_mmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
     if(rows <= 0) return HEFF_OK;
     const int64_t gx = cdiv(rows, ZM_TR), gy = cdiv(K, ZM_TK);
     if(gx > 0x7fffffff || gy > 65535) return HEFF_BAD_SHAPE;
-    HEFF_CUDA((launch_chained(z_slice_m_kernel<CPLX>, dim3((unsigned)gx, (unsigned)gy), ZM_THREADS, 0, s, src, rows, K, ld, p.inv, p.planes, p.kx, p.nslice, bad)));
+    HEFF_CUDA((launch_chained(z_slice_m_kernel<CPLX>, dim3((unsigned)gx, (unsigned)gy), ZM_THREADS, 0, s, src, rows, K, ld, p.inv, p.planes, p.ld, p.nslice, bad)));
     return HEFF_OK;
 }
 
@@ -560,10 +560,10 @@ __global__ void __launch_bounds__(ZCfg<BN>::THREADS, 1)
 }
 
 // CTA pair on a tile of 256 x 256 (tcgen05 cta_group::2): each CTA holds 128 rows of A and 128 of the tile's 256 rows of B, so a
-// k-block brings 32 KB into an SM for the same 128 x 256 x 128 products that a lone CTA needs 48 KB for, and what an SM can take
-// in (about 54 B/clk) bounds the main loop: the products of a real chi = 1000 matvec without their epilogue take 398 and 247 us by
-// lone CTAs and 290 and 211 by pairs (181 at the pipe's rate).  With it 599 and 335 before, 435 and 293 now: the levels summed in
-// C share that intake.
+// k-block brings 32 KB into an SM for the same 128 x 256 x 128 products that a lone CTA needs 48 KB for.  The products of a real
+// chi = 1000 matvec without their epilogue take 398 and 247 us by lone CTAs and 290 and 211 by pairs (181 at the pipe's rate).
+// With it 599 and 335 before, 417 and 293 now: in the first (K = 1000, short levels) the issuer waits 40 % of the time for
+// operands, which share the way from L2 with the levels summed in C.
 // Same roles as above; the even CTA's warp 1 issues the MMAs of both.  Its full barriers count both CTAs' bytes and its acc_empty
 // both CTAs' epilogue threads; commits arrive in both CTAs.
 constexpr uint32_t Z_IDESC_PAIR = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(2 * Z_BM >> 4) << 24);
@@ -746,10 +746,10 @@ int make_tmap_planes(CUtensorMap *map, const ZPlanes &p, int box_rows) {
         set_last_error_msg("cuTensorMapEncodeTiled is not available from the driver");
         return HEFF_CUDA_ERROR;
     }
-    if(((uintptr_t)p.planes & 15) || p.kx % 16 || p.rows <= 0 || p.nslice <= 0 || p.nslice > Z_MAX_SLICES) return HEFF_BAD_ARG;
+    if(((uintptr_t)p.planes & 15) || p.kx % 16 || p.ld % 16 || p.ld < p.kx || p.rows <= 0 || p.nslice <= 0 || p.nslice > Z_MAX_SLICES) return HEFF_BAD_ARG;
     std::memset(map, 0, sizeof(*map));
     cuuint64_t dims[3]    = {(cuuint64_t)p.kx, (cuuint64_t)p.rows, (cuuint64_t)p.nslice};
-    cuuint64_t strides[2] = {(cuuint64_t)p.kx, (cuuint64_t)(p.kx * p.rows)};
+    cuuint64_t strides[2] = {(cuuint64_t)p.ld, (cuuint64_t)(p.ld * p.rows)};
     cuuint32_t box[3]     = {(cuuint32_t)Z_BK, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3]    = {1, 1, 1};
     CUresult   r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, p.planes, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -779,12 +779,12 @@ static int z_forced_bn() {
 int z_choose_bn(int64_t M, int64_t N, int64_t K) {
     if(const int forced = z_forced_bn(); forced >= 128) return forced;
     // cost = waves x width x per-MAC weight (the 256-wide tile is a CTA pair's, two rows of tiles at once).  The weights are
-    // measured (7 slices, the real matvec GEMMs of chi = 1000, us at 256 / 192 / 128: K = 1000 435 / 535 / 533, K = 3000
-    // 293 / 520 / 535): the pair moves the least operand data, and the 128-wide tile's level sum in TMEM pays for short K only.
+    // measured (7 slices, the real matvec GEMMs of chi = 1000, us at 256 / 192 / 128: K = 1000 417 / 454 / 452, K = 3000
+    // 293 / 454 / 452): the pair moves the least operand data, and the 128-wide tile's level sum in TMEM pays for short K only.
     const int64_t sms  = device_sm_count();
     const int64_t kbs  = cdiv(K, Z_BK);
     const int     bn[3] = {256, 192, 128};
-    const double  w[3]  = {1.0, 1.2, kbs <= 8 ? 1.2 : 1.8};
+    const double  w[3]  = {1.0, 1.08, kbs <= 8 ? 1.08 : 1.5};
     int           best = 256;
     double        bc   = 1e300;
     for(int i = 0; i < 3; i++) {
@@ -921,13 +921,13 @@ static int gemm_emu_impl(const void *Av, const void *Bv, void *C, int64_t M, int
     }
     if(M > 0x7fffffff || cf * N > 0x7fffffff) return HEFF_BAD_SHAPE;
     auto          up    = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t  bPA   = up((size_t)ns * M * kx), bPB = up((size_t)ns * cf * N * kx);
+    const size_t  bPA   = up((size_t)ns * M * z_ld(kx)), bPB = up((size_t)ns * cf * N * z_ld(kx));
     const size_t  bS    = up(sizeof(double) * (size_t)(2 * M + 2 * N)), bE = 256;
     unsigned char *w    = nullptr;
     HEFF_TRY(stream_workspace(s, bPA + bPB + bS + bE, reinterpret_cast<void **>(&w)));
     ZPlanes pa, pb;
-    pa.planes = reinterpret_cast<int8_t *>(w), pa.rows = M, pa.kx = kx, pa.nslice = ns;
-    pb.planes = reinterpret_cast<int8_t *>(w + bPA), pb.rows = cf * N, pb.kx = kx, pb.nslice = ns;
+    pa.planes = reinterpret_cast<int8_t *>(w), pa.rows = M, pa.kx = kx, pa.ld = z_ld(kx), pa.nslice = ns;
+    pb.planes = reinterpret_cast<int8_t *>(w + bPA), pb.rows = cf * N, pb.kx = kx, pb.ld = z_ld(kx), pb.nslice = ns;
     double *sc = reinterpret_cast<double *>(w + bPA + bPB);
     pa.inv = sc, pa.fac = sc + M, pb.inv = sc + 2 * M, pb.fac = sc + 2 * M + N;
     int *err = reinterpret_cast<int *>(w + bPA + bPB + bS);  // err, bad word of A, bad word of B

@@ -55,10 +55,10 @@ struct ZPair {  // 256 x 256 tiles by CTA pairs
 constexpr int Z_MAX_SLICES  = 8;
 constexpr int Z_DEFAULT_SLICES = 7;
 
-// Digit planes of one operand: planes[t * rows * kx + r * kx + k], t < nslice; kx a multiple of 16 bytes.
+// Digit planes of one operand: planes[(t * rows + r) * ld + k], t < nslice, k < kx; kx and the pitch ld multiples of 16 bytes.
 struct ZPlanes {
     int8_t  *planes = nullptr;
-    int64_t  rows = 0, kx = 0;
+    int64_t  rows = 0, kx = 0, ld = 0;
     int      nslice = 0;
     double  *inv = nullptr;  // per source row: 64 / sigma_r (the first digit's scale)
     double  *fac = nullptr;  // per source row: sigma_r times the operand's extra factor (2^-12 on the A side)
@@ -96,8 +96,11 @@ int z_slice_kmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
 template<bool CPLX>
 int z_slice_mmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K, int64_t ld, const ZPlanes &p, int *bad, cudaStream_t s);
 
-// Plane row pitch for K source columns: round16(K), doubled for complex.
+// Plane row length for K source columns: round16(K), doubled for complex.
 inline int64_t z_kx(int64_t K, bool cplx) { return ((K + 15) / 16 * 16) * (cplx ? 2 : 1); }
+// Row pitch of a plane: whole 128-byte lines for rows of some length, so a 128-byte piece of a row is one line for L2 and not
+// two (real chi = 1000 GEMM 1, K = 1000, us at 256 / 192 / 128 columns: packed 435 / 535 / 533, whole lines 417 / 454 / 452).  Short rows stay packed: they would grow by more than a seventh.
+inline int64_t z_ld(int64_t kx) { return kx >= 896 ? (kx + 127) / 128 * 128 : kx; }
 // Largest K' for which no level sum can overflow INT32 (|d| <= 64, s slices folded per level).
 inline bool z_k_ok(int64_t kx, int nslice) { return kx > 0 && (int64_t)4096 * nslice * kx < ((int64_t)1 << 31); }
 

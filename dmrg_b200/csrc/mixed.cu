@@ -443,9 +443,9 @@ static int mixed_setup(heff_op *op) {
     HEFF_CUDA((launch_chained(split_L_kernel<CPLX>, g1(m->K1 * m->M1), 256, 0, s, reinterpret_cast<const T *>(op->L), m->A1, d.cL, m->M1, m->Kp1, m->Kx1)));
     HEFF_CUDA((launch_chained(split_R_kernel<CPLX>, g1(m->K2 * m->N2), 256, 0, s, reinterpret_cast<const T *>(op->Rp), m->B2, m->K2, d.cR, m->Kp2, m->Kx2)));
     HEFF_TRY(make_tmap_bf16(&m->tA1, m->A1, m->M1, m->Kx1, m->Kx1, X_BM));
-    HEFF_TRY(make_tmap_bf16(&m->tB1, m->B1, cf * m->N1, m->Kx1, m->Kx1, X_BN));
+    HEFF_TRY(make_tmap_bf16(&m->tB1, m->B1, cf * m->N1, m->Kx1, m->Kx1, X_BOX_B));
     HEFF_TRY(make_tmap_bf16(&m->tA2, m->A2, m->M2, m->Kx2, m->Kx2, X_BM));
-    HEFF_TRY(make_tmap_bf16(&m->tB2, m->B2, cf * m->N2, m->Kx2, m->Kx2, X_BN));
+    HEFF_TRY(make_tmap_bf16(&m->tB2, m->B2, cf * m->N2, m->Kx2, m->Kx2, X_BOX_B));
 
     m->wl_bytes = (int)wlist_bytes((int)d.DL, (int)d.DR, (int)d.S, sizeof(T));
     HEFF_CUDA((launch_chained(wlist_global_kernel<T>, 1, 32, 0, s, reinterpret_cast<const T *>(op->W), (int)d.DL, (int)d.DR, (int)d.S, m->wl)));
