@@ -66,13 +66,14 @@ static const TileShape &tile_shape(int cfg) {
 // Plan of one problem: the smallest estimate over tile shapes and K splits.  An SM does 64 DMMA FMAs per clock
 // whatever the tile, so a variant's time is the busiest SM's share of the padded products at the rate its tile sustains
 // (tile_shape), plus what its launches cost.  The constants come from a sweep of every variant over the matvec and
-// environment GEMMs of chi = 8 .. 1024 (real / complex): a GEMM of one k-tile takes 4.2 us back to back, a cluster of 2
-// or 4 adds 3.6 us (8 adds 7 and never won), the reduction kernel of a tail split 5 us.  Examples, us for (whole tiles
+// environment GEMMs of chi = 8 .. 1024 (real / complex): a cluster of 2 or 4 adds 3.6 us (8 adds 7 and never won), the chained
+// reduction kernel of a tail split 3 us (at 5, its price as a plain launch, whole tiles were kept too long: real S = 4
+// 313 x 569 178 / 154 us, S = 2 307 x 525 92 / 88).  Examples, us for (whole tiles
 // of 128/64/32 | best): f64 96x128x32 10.3/6.2/4.2 | 4.2; f64 1024x256x768 109/31/18.5 | 18.5; c128 192x128x384
 // -/49/18.5 | 10.3 (cluster of 4); f64 3072x4096x1024 840/-/- | 743 (tail split).
 template<bool CPLX>
 static GemmPlan gemm_pick(const GemmArgs &a) {
-    constexpr double kClk = 1.9e9, kLaunch = 3.2e-6, kCluster = 3.6e-6, kReduce = 5e-6, kHbm = 6.0e12;
+    constexpr double kClk = 1.9e9, kLaunch = 3.2e-6, kCluster = 3.6e-6, kReduce = 3e-6, kHbm = 6.0e12;
     const int     mode = split_mode(), sms = device_sm_count();
     const double  fma  = CPLX ? 3.0 : 1.0;
     GemmPlan      best;

@@ -779,12 +779,12 @@ static int z_forced_bn() {
 int z_choose_bn(int64_t M, int64_t N, int64_t K) {
     if(const int forced = z_forced_bn(); forced >= 128) return forced;
     // cost = waves x width x per-MAC weight (the 256-wide tile is a CTA pair's, two rows of tiles at once).  The weights are
-    // measured (7 slices, the real matvec GEMMs of chi = 1000, us at 256 / 192 / 128: K = 1000 417 / 454 / 452, K = 3000
-    // 293 / 454 / 452): the pair moves the least operand data, and the 128-wide tile's level sum in TMEM pays for short K only.
+    // measured (7 slices, the real matvec GEMMs of chi = 1000, us at 256 / 192 / 128: K = 1000 417 / 424 / 454, K = 3000
+    // 296 / 464 / 450): the pair moves the least operand data, and the 128-wide tile's level sum in TMEM pays for short K only.
     const int64_t sms  = device_sm_count();
     const int64_t kbs  = cdiv(K, Z_BK);
     const int     bn[3] = {256, 192, 128};
-    const double  w[3]  = {1.0, 1.08, kbs <= 8 ? 1.08 : 1.5};
+    const double  w[3]  = {1.0, 1.03, kbs <= 8 ? 1.09 : 1.5};
     int           best = 256;
     double        bc   = 1e300;
     for(int i = 0; i < 3; i++) {

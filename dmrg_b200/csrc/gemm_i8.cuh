@@ -99,7 +99,7 @@ int z_slice_mmajor(const typename Scalar<CPLX>::T *src, int64_t rows, int64_t K,
 // Plane row length for K source columns: round16(K), doubled for complex.
 inline int64_t z_kx(int64_t K, bool cplx) { return ((K + 15) / 16 * 16) * (cplx ? 2 : 1); }
 // Row pitch of a plane: whole 128-byte lines for rows of some length, so a 128-byte piece of a row is one line for L2 and not
-// two (real chi = 1000 GEMM 1, K = 1000, us at 256 / 192 / 128 columns: packed 435 / 535 / 533, whole lines 417 / 454 / 452).  Short rows stay packed: they would grow by more than a seventh.
+// two (real chi = 1000 GEMM 1, K = 1000, us at 256 / 192 / 128 columns: packed 435 / 535 / 533, whole lines 417 / 424 / 454).  Short rows stay packed: they would grow by more than a seventh.
 inline int64_t z_ld(int64_t kx) { return kx >= 896 ? (kx + 127) / 128 * 128 : kx; }
 // Largest K' for which no level sum can overflow INT32 (|d| <= 64, s slices folded per level).
 inline bool z_k_ok(int64_t kx, int nslice) { return kx > 0 && (int64_t)4096 * nslice * kx < ((int64_t)1 << 31); }
