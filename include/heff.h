@@ -294,7 +294,7 @@ int heff_gemm_i8_emu(int dtype, const void *A, const void *B, void *C, int64_t M
  * setting, or -1 for an invalid value.  Process-wide tuning knob; no counterpart
  * in the reference. */
 int heff_i8_set_tile_width(int bn);
-/* Kernels launched so far by the FP64 matvec path (its permutation and MPO mix) and by every DMMA
+/* Kernels launched so far by the FP64 matvec path (its fused kernel, or its permutation and MPO mix) and by every DMMA
  * GEMM (with its tail-split reduction), graph replays included, process-wide; read it around a
  * timed region of matvecs to count their launches.  No counterpart in the reference. */
 int64_t heff_matvec_launches(void);
@@ -304,8 +304,9 @@ int heff_i8_tuned_shapes(void);
 /* Tail split of the FP64 (DMMA) GEMMs of the matvec: when a GEMM's tiles leave
  * the last wave of the device partly empty, the tiles of that wave are split
  * along K into pieces whose partial tiles a second kernel sums in piece order.
- * mode 0 = off, 1 = automatic (a cost model of waves, partial traffic and the
- * extra launch; default), 2..16 = that many pieces whenever a wave is partial.
+ * mode 0 = off (no K split of any kind), 1 = automatic (a cost model of waves,
+ * partial traffic and the extra launch, which may take smaller tiles or a K split
+ * over a cluster of CTAs instead; default), 2..16 = that many pieces whenever a wave is partial.
  * The initial value comes from the environment variable HEFF_GEMM_SPLIT.  Results
  * are deterministic for a given mode and device but differ from the unsplit
  * product at the rounding level.  Returns the previous mode, or -1 for an invalid
