@@ -31,10 +31,35 @@ int check_matvec_dims(const int64_t md[3], const int64_t wd[4], const int64_t ld
     return HEFF_OK;
 }
 
-// x'[a + cL*(s + S*b)] = x[s + S*(a + cL*b)]   (output-linear: coalesced writes)
+// x'[a + cL*(s + S*b)] = x[s + S*(a + cL*b)].  For the spins of one and two sites a thread moves the S values of a point (a, b),
+// 16 bytes a load where x allows it, into S streams of consecutive a: one division per point, and whole sectors on both sides.
+// Other spins go output-linear, one value and two divisions per thread.  us, output-linear / by points: real S = 4
+// 1000 x 1000 20.0 / 10.9, 367 x 251 5.7 / 4.0, complex S = 4 1024 x 1024 25.5 / 17.8.
+template<class T, int S>
+__device__ __forceinline__ void permute_points(const T *__restrict__ x, T *__restrict__ xp, int64_t cL, int64_t points) {
+    const bool vec = sizeof(T) == 8 && ((uintptr_t)x & 15u) == 0;
+    for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < points; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t b = points <= 0x7fffffff ? (int64_t)((unsigned)e / (unsigned)cL) : e / cL, a = e - cL * b;
+        T             v[S];
+        if(vec) {
+#pragma unroll
+            for(int s = 0; s < S; s += 2) {
+                const double2 w = *reinterpret_cast<const double2 *>(x + S * e + s);
+                *reinterpret_cast<double *>(&v[s]) = w.x, *reinterpret_cast<double *>(&v[s + 1]) = w.y;
+            }
+        } else {
+#pragma unroll
+            for(int s = 0; s < S; s++) v[s] = x[S * e + s];
+        }
+#pragma unroll
+        for(int s = 0; s < S; s++) xp[a + cL * (s + S * b)] = v[s];
+    }
+}
 template<class T>
 __global__ void permute_mps_kernel(const T *__restrict__ x, T *__restrict__ xp, int64_t S, int64_t cL, int64_t n) {
     grid_wait();
+    if(S == 4) return permute_points<T, 4>(x, xp, cL, n / 4);
+    if(S == 2) return permute_points<T, 2>(x, xp, cL, n / 2);
     for(int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t a = o % cL, r = o / cL, s = r % S, b = r / S;
         xp[o]           = x[s + S * (a + cL * b)];
