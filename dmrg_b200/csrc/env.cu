@@ -17,6 +17,7 @@ namespace heff {
 
 __device__ __forceinline__ double conj_s(double v) { return v; }
 __device__ __forceinline__ double2 conj_s(double2 v) { return make_double2(v.x, -v.y); }
+
 // Mc[a' + cL*(s' + d*b')] = conj(M[s' + d*(a' + cL*b')])
 template<class T>
 __global__ void env_prep_L(const T *__restrict__ M, T *__restrict__ Mc, int64_t d, int64_t cL, int64_t n) {
