@@ -443,6 +443,7 @@ __global__ void __launch_bounds__(JTHR) jacobi_round_kernel(T *__restrict__ G, i
                                                            int round, double tol, double floor_abs, const int *__restrict__ colmap,
                                                            double *__restrict__ gmax_out, int *__restrict__ rotated, int CL) {
     grid_wait();
+    if(CL > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");  // met before the first remote store
     using S  = JS<T>;
     using JK = JPairBlock<T>;
     constexpr int RC = S::ROWS;
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(JTHR) jacobi_round_kernel(T *__restrict__ G, i
 #pragma unroll
             for(int u = 0; u < 4; u++) mine[JK::row(k, u) * JK::LD + JK::col(k, u)] = JK::make(re[0][k][u] + re[1][k][u], im[0][k][u] + im[1][k][u]);
         __syncthreads();
+        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // every CTA has started: its shared memory may be written
         constexpr int PC = S::PER_COPY;  // 16 bytes a store, whole rows in order
         for(int r = 1; r < CL; r++) {
             const int to  = (rank + r) % CL;
@@ -830,6 +832,7 @@ struct QrPanel {
 template<class T>
 __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T *__restrict__ G, int64_t ldg, int M, int j0, int w, T *__restrict__ Tout, int CL) {
     grid_wait();
+    if(CL > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");  // met before the first remote store
     using S           = JS<T>;
     constexpr int RPT = QrPanel<T>::RPT;
     __shared__ T      s_red[QrPanel<T>::THR_MAX / 32][QW];
@@ -885,6 +888,7 @@ __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T
         if(CL > 1) {
             namespace cg = cooperative_groups;
             cg::cluster_group cluster = cg::this_cluster();
+            if(j == 0) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // every CTA has started
             if(ctl && lane < QW)
                 for(int q = 0; q < CL; q++) {
                     T *dst    = cluster.map_shared_rank(&s_cl[j & 1][rank][0], q);
