@@ -104,7 +104,9 @@ __device__ __forceinline__ void zero(double2 &v) { v = make_double2(0.0, 0.0); }
 // A zero weight must not touch its input: the reference skips zero entries, and 0 * inf would not.  A warp that meets a
 // non-finite input computes its points entry by entry instead (mix_skip).
 // us before / after: chi = 16 real D = 3 10.6 / 5.2, chi = 1024 complex D = 3 114 / 89 (HBM floor 62), real D = 9 367 x 251
-// 53 / 26, environment real D = 9 640 x 517 165 / 43.
+// 53 / 26, environment real D = 9 640 x 517 165 / 43 Larger MPOs too, whole product, real 256 x 256, from the nonzero list / dense:
+// S = 16 D = 3 (72 fragments of W) 247 / 156, S = 4 D = 16 (128) 387 / 191, S = 8 D = 9 (162) 430 / 221; complex S = 16 D = 3
+// 559 / 448.
 template<class T>
 __device__ __noinline__ void mix_skip(const MixArgs &a, const T *tile, int pitch, int p, int q, int o0, int o1) {
     const int S = a.S, NI = a.K * S;
@@ -258,27 +260,39 @@ __global__ void __launch_bounds__(2 * TP) mix_dense_kernel(const MixArgs a) {
     }
 }
 
-// Entry by entry from global memory: MPO bonds whose dense product would not pay (more than MIX_DENSE fragments) or whose
-// tiles do not fit.  One thread per point, W's entries by uniform loads.
+// Entry by entry: environment MPOs whose input rows do not fit a tile of 32 points (K S of about 700 real, 300 complex and more).
+// One thread per point, bound by the chain of its loads; W in shared memory, in the order of the sum, so an entry costs a load and
+// a test (read from global memory and its indices by division: environment d = 2 1024 -> 1 at chi = 64 936 us, now 457).
+constexpr size_t MIX_SMEM = 200 * 1024;
 template<class T>
 __global__ void __launch_bounds__(128) mix_entry_kernel(const MixArgs a) {
     grid_wait();
-    const int S = a.S, NI = a.K * S;
-    const T  *W = reinterpret_cast<const T *>(a.W);
+    extern __shared__ __align__(16) unsigned char mix_smem[];
+    T            *sW = reinterpret_cast<T *>(mix_smem);  // (output, input)
+    const T      *W  = reinterpret_cast<const T *>(a.W);
+    const int     S = a.S, NI = a.K * S, NO = a.J * S;
+    const int     n1 = a.s_fastest ? a.K : S, n2 = a.s_fastest ? S : a.K;  // outer and inner index of the sum
+    const int64_t d1 = a.s_fastest ? a.in_k : a.in_s, d2 = a.s_fastest ? a.in_s : a.in_k;
+    for(int e = threadIdx.x; e < NI * NO; e += blockDim.x) {
+        const int o = e / NI, i = e - o * NI, j = o / S, so = o - j * S, i1 = i / n2, i2 = i - i1 * n2;
+        const int k = a.s_fastest ? i1 : i2, s = a.s_fastest ? i2 : i1;
+        sW[e] = W[(int64_t)a.w_k * k + (int64_t)a.w_j * j + (int64_t)a.w_s * s + (int64_t)a.w_so * so];
+    }
+    __syncthreads();
     for(int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)a.P * a.nq; e += (int64_t)gridDim.x * blockDim.x) {
         const int p = (int)(e % a.P), q = a.q0 + (int)(e / a.P);
-        const T  *x = reinterpret_cast<const T *>(a.in) + p + a.in_q * q;
-        T        *o = reinterpret_cast<T *>(a.out) + (int64_t)S * (p + (int64_t)a.P * q);
+        const T  *x = reinterpret_cast<const T *>(a.in) + p + a.in_q * q, *w = sW;
+        T        *out = reinterpret_cast<T *>(a.out) + (int64_t)S * (p + (int64_t)a.P * q);
         for(int j = 0; j < a.J; j++)
             for(int so = 0; so < S; so++) {
                 T acc;
                 zero(acc);
-                for(int i = 0; i < NI; i++) {
-                    const int k = a.s_fastest ? i / S : i % a.K, s = a.s_fastest ? i % S : i / a.K;
-                    const T   w = __ldg(W + (int64_t)a.w_k * k + (int64_t)a.w_j * j + (int64_t)a.w_s * s + (int64_t)a.w_so * so);
-                    if(!is_zero(w)) acc = fma_s(w, x[a.in_k * k + a.in_s * s], acc);
+                for(int i1 = 0; i1 < n1; i1++) {
+                    const T *xi = x + d1 * i1;
+                    for(int i2 = 0; i2 < n2; i2++, w++)
+                        if(!is_zero(*w)) acc = fma_s(*w, xi[d2 * i2], acc);
                 }
-                o[so + (int64_t)S * a.P * a.Q * j] = acc;
+                out[so + (int64_t)S * a.P * a.Q * j] = acc;
             }
     }
 }
@@ -288,7 +302,6 @@ static size_t mix_bytes(const MixArgs &a, int bufs) {
     const size_t KS = (size_t)cdiv((int64_t)a.K * a.S, 4), NT = (size_t)cdiv((int64_t)a.J * a.S, 8);
     return sizeof(T) * (bufs * 4 * KS * MixTile<T, TP>::PITCH + KS * NT * 32);
 }
-constexpr size_t MIX_SMEM = 200 * 1024;
 template<class T, int TP, int NTC>
 static int mix_launch(const MixArgs &a, cudaStream_t s) {
     const size_t smem = mix_bytes<T, TP>(a, a.bufs);
@@ -313,17 +326,18 @@ static int mix_tiles(MixArgs a, cudaStream_t s) {
     return cdiv((int64_t)a.J * a.S, 8) <= 2 ? mix_launch<T, TP, 2>(a, s) : mix_launch<T, TP, 5>(a, s);
 }
 // Points per tile: 128, fewer while that leaves SMs without a CTA or the tile does not fit.
-constexpr int64_t MIX_DENSE = 64;  // DMMA fragments of W up to which the dense product is taken (D = 9, S = 4 has 45)
 template<bool CPLX>
 int mpo_mix(MixArgs a, cudaStream_t s) {
     using T = typename Scalar<CPLX>::T;
     if(a.nq <= 0 || a.P <= 0) return HEFF_OK;
     a.pairs = !CPLX && a.S % 2 == 0 && ((uintptr_t)a.out & 15u) == 0;
     a.vec   = !CPLX && ((uintptr_t)a.in & 15u) == 0 && a.P % 2 == 0 && a.in_k % 2 == 0 && a.in_s % 2 == 0 && a.in_q % 2 == 0;
-    const int64_t frags = cdiv((int64_t)a.K * a.S, 4) * cdiv((int64_t)a.J * a.S, 8);
-    if(frags > MIX_DENSE || mix_bytes<T, 32>(a, 1) > MIX_SMEM) {
+    if(mix_bytes<T, 32>(a, 1) > MIX_SMEM) {
+        const size_t  wsm = sizeof(T) * (size_t)a.K * a.J * a.S * a.S;
         const int64_t n = (int64_t)a.P * a.nq, g = std::min<int64_t>(cdiv(n, 128), (int64_t)device_sm_count() * 16);
-        HEFF_CUDA((launch_chained(mix_entry_kernel<T>, (unsigned)g, 128, 0, s, a)));
+        if(wsm > MIX_SMEM) return HEFF_BAD_SHAPE;  // neither operators nor environments accept such an MPO
+        if(wsm > 48 * 1024) HEFF_CUDA(cudaFuncSetAttribute(mix_entry_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MIX_SMEM));
+        HEFF_CUDA((launch_chained(mix_entry_kernel<T>, (unsigned)g, 128, wsm, s, a)));
         return HEFF_OK;
     }
     auto padded = [&](int tp) { return cdiv(a.P, tp) * tp; };
