@@ -1,6 +1,7 @@
 // H_eff * theta: layout kernels, MPO mixing kernel, matvec driver, expectation value,
 // and the stateless C entry points heff_matvec_{d,z} / heff_expval_{d,z}.
 #include <algorithm>
+#include <initializer_list>
 #include "matvec.cuh"
 #include "runtime.cuh"
 #include "wlist.cuh"
@@ -633,6 +634,17 @@ template int dot_device<false>(const double *, const double *, int64_t, double *
 template int dot_device<true>(const double2 *, const double2 *, int64_t, double2 *, double *, cudaStream_t);
 
 // ---- stateless entry points ----
+// Complex tensors are read by 16-byte loads on every route (the GEMM refuses others, the one-launch product has no such test).
+template<bool CPLX>
+static int check_alignment(std::initializer_list<const void *> tensors) {
+    for(const void *p : tensors)
+        if(CPLX && ((uintptr_t)p & 15u)) {
+            set_last_error_msg("matvec: complex tensors must be 16-byte aligned");
+            return HEFF_BAD_ARG;
+        }
+    return HEFF_OK;
+}
+
 template<bool CPLX>
 static int matvec_stateless(void *res, const void *mps, const int64_t md[3], const void *mpo, const int64_t wd[4], const void *envL,
                             const int64_t ld[3], const void *envR, const int64_t rd[3], cudaStream_t s) {
@@ -644,6 +656,7 @@ static int matvec_stateless(void *res, const void *mps, const int64_t md[3], con
         set_last_error_msg("matvec: res must not alias mps");
         return HEFF_BAD_ARG;
     }
+    HEFF_TRY(check_alignment<CPLX>({res, mps, mpo, envL, envR}));
     if(matvec_fused_fits<CPLX>(d)) {  // R in the caller's layout
         if(mpo_too_large<CPLX>(d)) return HEFF_BAD_SHAPE;
         return matvec_fused<CPLX>(d, reinterpret_cast<const T *>(mps), reinterpret_cast<T *>(res), reinterpret_cast<const T *>(envL),
@@ -669,6 +682,7 @@ static int expval_stateless(double *result, const void *mps, const int64_t md[3]
     MatvecDims d;
     HEFF_TRY(check_matvec_dims(md, wd, ld, rd, d));
     if(!result || !mps || !mpo || !envL || !envR) return HEFF_BAD_ARG;
+    HEFF_TRY(check_alignment<CPLX>({mps, mpo, envL, envR}));
     const int64_t extra = MatvecScratch<CPLX>::pad(d.size_Rp()) + MatvecScratch<CPLX>::pad(d.size_mps()) + 1;
     const int64_t elems = MatvecScratch<CPLX>::elems(d) + extra;
     void         *base  = nullptr;
