@@ -117,11 +117,6 @@ __device__ __forceinline__ void dmma_f64(double (&c)[4], double a0, double a1, d
                  : "d"(a0), "d"(a1), "d"(b0));
 }
 
-__device__ __forceinline__ float sqrt_fast(float x) {
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ float rcp_fast(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -148,13 +143,11 @@ __device__ __forceinline__ bool significant(double a, double b, double2 apq, dou
     return h2 > fl * fl && h2 > tol * tol * fabs(a * b);
 }
 
-// Rotation that annihilates apq = |apq| e in the Hermitian 2x2 block [[app, apq], [conj(apq), aqq]]: p = s tan(angle / 2)
-// and se = s e, false when apq is not significant.  The angle and the phase need only be right to single precision (what
-// remains of apq is 1e-7 of it, left to the next sweep); the rotation must be unitary to double precision.  So half-angle
-// tangents u and v come from single precision, and the rational forms s = 2 u / (1 + u^2), p = s u,
-// e = +-((1 - v^2) + 2 i v) / (1 + v^2) are unitary for any u and v: one short Newton reciprocal each in place of a chain of
-// divisions and square roots.  With x = (aqq - app) / 2, w = sqrt(x^2 + h^2), y = |x| + w: tan(angle) = h / y and
-// u = h / (y + sqrt(2 w y)).
+// Rotation that annihilates apq = |apq| e in the Hermitian 2x2 block [[app, apq], [conj(apq), aqq]]: p = 1 - cos and se = e sin
+// of its angle, false when apq is not significant.  All in double precision and without a division: with x = (aqq - app) / 2,
+// h = |apq| and w = sqrt(x^2 + h^2), |x| / w is the cosine of twice the angle and h / w its sine; the half-angle formulas give
+// c = sqrt((1 + |x| / w) / 2) and s = h / (2 w c).  p = s^2 / (1 + c) is as right as s is, so (1 - p)^2 + s^2 = 1 holds to s^2 eps
+// for tiny angles too, where 1 - c would have lost p.
 template<class T>
 __device__ __forceinline__ bool jacobi_rotation(double app, double aqq, T apq, double tol, double floor_abs, double &p, T &se) {
     const double sc = pair_scale(app, aqq), a = app * sc, b = aqq * sc, fl = floor_abs * sc;
@@ -162,39 +155,33 @@ __device__ __forceinline__ bool jacobi_rotation(double app, double aqq, T apq, d
     p  = 0.0;
     se = JS<T>::zero();
     if(!significant(a, b, z, tol, fl)) return false;
-    const float xf = (float)(0.5 * (b - a));
-    float       h, sg;  // apq = sg h e
-    T           e{};
+    const double x = 0.5 * (b - a), h2 = JS<T>::abs2(z);
+    const double rw = rsqrt(fma(x, x, h2)), v = fma(0.5 * fabs(x), rw, 0.5), rc = rsqrt(v);  // v = c^2
+    const double q = copysign(0.5 * rw * rc, x), rd = rcp_near_one(fma(v, rc, 1.0));
+    double       sn;
     if constexpr(std::is_same<T, double>::value) {
-        h  = fabsf((float)z);
-        sg = z < 0.0 ? -1.0f : 1.0f;
-        e  = 1.0;
+        se = z * q;
+        sn = se;
     } else {
-        const float rf = (float)z.x, mf = (float)z.y;
-        sg = rf < 0.0f ? -1.0f : 1.0f;
-        const float mx = fmaxf(fabsf(rf), fabsf(mf)), q = mx > 0.0f ? fminf(fabsf(rf), fabsf(mf)) * rcp_fast(mx) : 0.0f;
-        h  = mx * sqrt_fast(fmaf(q, q, 1.0f));  // the squares of an |apq| below 1e-19 would leave single precision's range
-        const double v = h > 0.0f ? (double)(mf * sg * rcp_fast(h + fabsf(rf))) : 0.0, rv = rcp_near_one(fma(v, v, 1.0));
-        e              = make_double2(fma(-v, v, 1.0) * rv, 2.0 * v * rv);
+        se = JS<T>::scale(z, q);
+        sn = h2 * rsqrt(h2) * q;
     }
-    const float w = sqrt_fast(fmaf(xf, xf, h * h)), y = fabsf(xf) + w;
-    double      u = (double)(h * rcp_fast(y + sqrt_fast(2.0f * w * y)));
-    if((xf < 0.0f) != (sg < 0.0f)) u = -u;
-    if(!(u != 0.0)) return false;  // below single precision's range: no rotation changes anything
-    const double sn = 2.0 * u * rcp_near_one(fma(u, u, 1.0));
-    p               = sn * u;
-    se              = JS<T>::scale(e, sn);
-    return true;
+    p = sn * sn * rd;
+    if(p > 0.0) return true;
+    se = JS<T>::zero();  // an angle below 1e-162 (or not a number): p = 0 says no rotation
+    p  = 0.0;
+    return false;
 }
-// x - p x - c y and x - p x + c y: a rotation's new columns, (1 - p) the cosine.  x - p x as one fused operation keeps the
-// rounding of the cosine (near 1 for tiny angles) from inflating every column it multiplies.
-__device__ __forceinline__ double  rot_sub(double x, double y, double c, double p) { return fma(-c, y, fma(-p, x, x)); }
-__device__ __forceinline__ double  rot_add(double x, double y, double c, double p) { return fma(c, y, fma(-p, x, x)); }
+// x - (p x + c y) and x - (p x - c y): a rotation's new columns, 1 - p its cosine.  The bracket is as small as the angle, so the
+// result takes one rounding of its own size (x - p x - c y from left to right takes two, complex three: orthogonality of the right
+// factor 13 % worse).
+__device__ __forceinline__ double  rot_sub(double x, double y, double c, double p) { return x - fma(p, x, c * y); }
+__device__ __forceinline__ double  rot_add(double x, double y, double c, double p) { return x - fma(p, x, -(c * y)); }
 __device__ __forceinline__ double2 rot_sub(double2 x, double2 y, double2 c, double p) {
-    return make_double2(fma(c.y, y.y, fma(-c.x, y.x, fma(-p, x.x, x.x))), fma(-c.y, y.x, fma(-c.x, y.y, fma(-p, x.y, x.y))));
+    return make_double2(x.x - fma(p, x.x, fma(c.x, y.x, -(c.y * y.y))), x.y - fma(p, x.y, fma(c.x, y.y, c.y * y.x)));
 }
 __device__ __forceinline__ double2 rot_add(double2 x, double2 y, double2 c, double p) {
-    return make_double2(fma(-c.y, y.y, fma(c.x, y.x, fma(-p, x.x, x.x))), fma(c.y, y.x, fma(c.x, y.y, fma(-p, x.y, x.y))));
+    return make_double2(x.x - fma(p, x.x, fma(-c.x, y.x, c.y * y.y)), x.y - fma(p, x.y, -fma(c.x, y.y, c.y * y.x)));
 }
 
 // Shared pieces of the two Jacobi kernels for P = 32 (a pair of blocks) or 64 columns on THR threads.  G and Q are P x P
@@ -279,8 +266,7 @@ struct JBlock {
     // rotations).  Only significant off-diagonals are rotated (half the convergence test's thresholds: the two triangles of
     // a Gram differ by rounding, and a pair that the test sees must rotate); a step without any costs one barrier.  Step s
     // pairs (nc - 1, s) and ((s + k) mod (nc - 1), (s - k) mod (nc - 1)): each thread advances its pairs by one instead of
-    // evaluating the remainders.  A step takes 0.5 us (P = 32, real): 490 clocks the rotations, 330 the blocks, 110 the
-    // barriers.
+    // evaluating the remainders.  A step takes 0.5 us (P = 32, real), most of it the chain of a rotation's operations.
     struct Pair {
         int a, b, fixed;
         __device__ Pair(int k, int nc) : a(k == 0 ? nc - 1 : k), b(k == 0 ? 0 : nc - 1 - k), fixed(k == 0) {}
