@@ -838,7 +838,7 @@ __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T
         for(int c = 0; c < QW; c++) a[i][c] = (!ctl && lr0 + i * thr < rows && c < w) ? G[(j0 + lr0 + i * thr) + ldg * (int64_t)(j0 + c)] : S::zero();
 
 #pragma unroll 1
-    for(int j = 0; j < QW; j++) {  // columns past w are zero and change nothing
+    for(int j = 0; j < w; j++) {  // registers of columns past w hold zeros and change nothing
         if(!ctl) {
             T d[QW];
 #pragma unroll
@@ -893,7 +893,7 @@ __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T
         if(ctl) {
             // v = (x - beta e_j) inv, v_j = 1; w_c = v^H a_c = conj(inv) (x^H a_c - beta a_jc); a_c -= conj(tau) w_c v
             const double sig2 = S::re(piv);
-            double beta = 0.0;
+            double beta = sig2;  // zero column: 0; a NaN stays one
             T      inv = S::zero(), g = S::zero(), f = S::zero();
             if(sig2 > 0) {
                 const double rs = rsqrt(sig2), nrm = sig2 * rs, ar = S::re(alpha);
@@ -971,8 +971,10 @@ __global__ void __launch_bounds__(QrPanel<T>::THR_MAX + 32, 1) qr_panel_kernel(T
 #pragma unroll
         for(int i = 0; i < RPT; i++)
 #pragma unroll
-            for(int c = 0; c < QW; c++)
-                if(lr0 + i * thr < rows && c < w) G[(j0 + lr0 + i * thr) + ldg * (int64_t)(j0 + c)] = a[i][c];
+            for(int c = 0; c < QW; c++) {
+                const int pc = (c + w) & (QW - 1);  // the columns have been rotated w times
+                if(lr0 + i * thr < rows && pc < w) G[(j0 + lr0 + i * thr) + ldg * (int64_t)(j0 + pc)] = a[i][c];
+            }
     } else if(rank == 0 && lane < QW) {
 #pragma unroll
         for(int c = 0; c < QW; c++) Tout[lane + QW * c] = a[0][c];
@@ -1117,6 +1119,20 @@ int64_t truncation_rank(const double *S, int64_t n, int64_t rank_max, int64_t ra
     return rank;
 }
 
+// Factorisations before Jacobi, for A in its tall orientation:
+//   2  A P = Q1 R1, R1^H = Q2 R2, Jacobi on R2^H;   1  A = Q1 R1 (one panel), Jacobi on R1;   0  Jacobi on A.
+// Both factorisations cost about 2.3 us a column and eight launches, and save sweeps, most on graded spectra; one factor alone
+// makes a long matrix short enough for shared memory.  us for none / one / both, Gaussian | graded: real 16 x 16 151 / - / 195 |
+// 222 / - / 230, 17 x 17 177 / - / 279 | 240 / - / 238, 32 x 32 252 / - / 317 | 490 / - / 278, 256 x 4 118 / 96 / - | 118 / 93 / -,
+// 300 x 8 187 / 121 / 154 | 200 / 132 / 137, 300 x 16 255 / 170 / 195 | 400 / 241 / 170; complex 256 x 16 342 / 245 / - |
+// 637 / 350 / -.  A panel of more than ROWS_MAX rows does not fit the registers of a cluster of eight CTAs.
+template<class T>
+static int svd_factors(int64_t M, int64_t N) {
+    if(M > QrPanel<T>::ROWS_MAX) return 0;
+    if(N > QW + 1 || (N > QW && M > JW_ROWS) || (N >= 10 && M > 256)) return 2;
+    return M > (N == 1 ? 256 : JW_ROWS) ? 1 : 0;
+}
+
 // In-place QR of G (M x N, leading dim ldg); the panels' T factors go to Tf (QW x QW each).
 template<class T>
 static int qr_factor(T *G, int64_t ldg, int M, int N, T *Tf, cudaStream_t s) {
@@ -1189,10 +1205,8 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
         HEFF_CUDA((launch_chained(col_order_kernel, (cols + 127) / 128, 128, 0, s, nrm, cols, ord)));
         return HEFF_OK;
     };
-    // Preconditioned from 17 columns on, and whenever the rows are many: measured on real 32 x 32 matrices, 0.39 ms with and
-    // 1.03 ms without on a graded spectrum, 0.45 and 0.48 ms on a Gaussian one; at 16 columns Jacobi's few short sweeps cost
-    // less than the two factorisations (0.19 ms as it is).
-    const bool precond = M <= QrPanel<T>::ROWS_MAX && (N > 16 || M > 256);
+    const int     qr   = svd_factors<T>(M, N);
+    const bool    precond = qr > 0;
     T            *W    = precond ? Y : G;  // the matrix Jacobi works on, rows x npad
     const int64_t ldw  = precond ? npad : ldg;
     const int     rows = precond ? N : M;
@@ -1200,20 +1214,25 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     const T      *src  = A;
     int64_t       lds  = lda;
     if(wide && (precond || !whole)) {
-        T *dst = precond ? Z : G;
-        HEFF_CUDA(cudaMemsetAsync(dst, 0, sizeof(T) * (size_t)ldg * npad, s));
+        T *dst = qr == 2 ? Z : G;
+        HEFF_CUDA(cudaMemsetAsync(dst, 0, sizeof(T) * (size_t)ldg * (qr == 1 ? QW : npad), s));  // a panel is read in whole
         HEFF_CUDA((launch_chained(adjoint_kernel<T, false>, dim3((unsigned)cdiv(N, 32), (unsigned)cdiv(M, 32)), 256, 0, s, A, lda, (int)m, (int)n, dst, ldg, M, N)));
         src = dst, lds = ldg;
     }
-    if(precond) {
+    const dim3 sq((unsigned)(npad / 32), (unsigned)(npad / 32));
+    if(qr == 2) {
         // G = A or A^H with the columns by descending norm: the factors of a matrix whose columns differ by orders of
         // magnitude keep each column's own relative accuracy, and zero columns come last
         HEFF_TRY(norms_order(src, lds, M, N, sig0, cord));
         HEFF_CUDA((launch_chained(copy_pad_kernel<T>, g1(ldg * npad), 256, 0, s, src, lds, M, N, G, ldg, npad, cord)));
         HEFF_TRY(qr_factor<T>(G, ldg, M, N, T1, s));
-        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, dim3((unsigned)(npad / 32), (unsigned)(npad / 32)), 256, 0, s, G, ldg, N, N, X, npad, npad, npad)));
+        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, sq, 256, 0, s, G, ldg, N, N, X, npad, npad, npad)));
         HEFF_TRY(qr_factor<T>(X, npad, N, N, T2, s));
-        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, dim3((unsigned)(npad / 32), (unsigned)(npad / 32)), 256, 0, s, X, npad, N, N, Y, npad, npad, npad)));
+        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, sq, 256, 0, s, X, npad, N, N, Y, npad, npad, npad)));
+    } else if(qr == 1) {  // a zero column stays exactly zero through the factorisation
+        if(!wide) HEFF_CUDA((launch_chained(copy_pad_kernel<T>, g1(ldg * QW), 256, 0, s, src, lds, M, N, G, ldg, QW, nullptr)));
+        HEFF_TRY(qr_factor<T>(G, ldg, M, N, T1, s));
+        HEFF_CUDA((launch_chained(adjoint_kernel<T, true>, sq, 256, 0, s, G, ldg, N, N, Y, npad, npad, npad)));  // R1^H
     } else if(!wide && !whole) {
         HEFF_CUDA((launch_chained(copy_pad_kernel<T>, g1(ldg * npad), 256, 0, s, src, lds, M, N, G, ldg, npad, nullptr)));
     }
@@ -1226,7 +1245,7 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     if(whole) {
         const T      *from = precond ? W : A;
         const int64_t ldf  = precond ? ldw : lda;
-        const int     adj  = !precond && wide;
+        const int     adj  = qr == 1 || (!precond && wide);
         if(npad == 32)
             HEFF_CUDA((launch_chained(jacobi_whole_kernel<T, 32>, 1, jw_thr(32), jacobi_whole_bytes<T, 32>(), s, from, ldf, adj, W, ldw, rows, N, V, tol, JOUTER, sig, drot)));
         else
@@ -1272,7 +1291,7 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return host[a] > host[b]; });
     std::vector<double> sorted(N);
     for(int i = 0; i < N; i++) sorted[i] = host[order[i]];
-    if(precond) {  // as many zero singular values as zero columns (the factorisation leaves rounding noise in their place)
+    if(qr == 2) {  // as many zero singular values as zero columns (the factorisation leaves rounding noise in their place)
         int nzero = 0;
         for(int i = 0; i < N; i++) nzero += host[npad + 64 + i] == 0.0;
         for(int i = 0; i < nzero; i++) sorted[N - 1 - i] = 0.0;
@@ -1284,13 +1303,22 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     }
     *rank = r;
     HEFF_CUDA(cudaMemcpyAsync(perm, order.data(), sizeof(int) * r, cudaMemcpyHostToDevice, s));
-    // ---- singular vectors: left = Q1 [U_j; 0] (M x r), right = P Q2 V_j (N x r); U and VT, exchanged for a wide A
+    // ---- singular vectors: left = Q1 [U_j; 0] (M x r), right = P Q2 V_j or V_j (N x r); U and VT, exchanged for a wide A
     const int kk = (int)r, gr = g1((int64_t)(M + N) * r);
     if(!precond) {
         if(!wide)
             HEFF_CUDA((launch_chained(take_columns_kernel<T, false, true>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, U, M, M, VT, 0)));
         else
             HEFF_CUDA((launch_chained(take_columns_kernel<T, true, false>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, VT, 0, M, U, N)));
+    } else if(qr == 1) {
+        T            *left = wide ? Z : U;
+        const int64_t ldl  = wide ? ldg : M;
+        if(!wide)
+            HEFF_CUDA((launch_chained(take_columns_kernel<T, false, true>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, left, ldl, M, VT, 0)));
+        else
+            HEFF_CUDA((launch_chained(take_columns_kernel<T, false, false>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, left, ldl, M, U, N)));
+        HEFF_TRY(qr_apply_q<T>(G, ldg, M, N, T1, left, ldl, kk, s));
+        if(wide) HEFF_CUDA((launch_chained(adjoint_rows_kernel<T>, g1((int64_t)M * r), 256, 0, s, left, ldl, M, kk, nullptr, VT)));
     } else {
         T            *left = wide ? Z : U;
         const int64_t ldl  = wide ? ldg : M;
