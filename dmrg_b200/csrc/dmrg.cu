@@ -175,7 +175,7 @@ struct DmrgWorkspace {
         const size_t  big = (size_t)(d * (1 + Dcap) * chi * chi) + 64;
         for(double **p : {&eP, &eX, &eT, &eU, &eV, &eY, &eZ}) HEFF_TRY(get(p, big));
         const int64_t m = (1 + Dcap) * chi, n = d * chi;
-        HEFF_TRY(get(&escr, (size_t)(svd_scratch_bytes(m, n, 8) / 8) + 64));
+        HEFF_TRY(get(&escr, (size_t)(svd_scratch_max(m, n, 8) / 8) + 64));
         onesite = true;
         return HEFF_OK;
     }
@@ -219,7 +219,7 @@ struct DmrgWorkspace {
         HEFF_TRY(get(&S, (size_t)(2 * chi + 64)));
         HEFF_TRY(get(&V, tsz));
         const int64_t md_max[3] = {d, chi, chi}, wd_max[4] = {Dmax, Dmax, 2, 2};
-        const size_t  scr_elems = std::max<size_t>((size_t)env_scratch_elems(md_max, wd_max), (size_t)schmidt_scratch_bytes(d, d, chi, chi, chi) / 8 + 64);
+        const size_t  scr_elems = std::max<size_t>((size_t)env_scratch_elems(md_max, wd_max), (size_t)schmidt_scratch_max(d, d, chi, chi, chi) / 8 + 64);
         HEFF_TRY(get(&scr, scr_elems));
         HEFF_TRY(op_create_capacity(&op, false, d * d, chi, Dmax, prec, stream));
         if(engine == HEFF_FP64_INT8) {

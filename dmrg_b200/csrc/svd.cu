@@ -1087,16 +1087,6 @@ static int g1(int64_t n) {
     return (int)(g < 1 ? 1 : (g < cap ? g : cap));
 }
 
-// Scratch of one SVD, in its tall orientation (M = max, N = min of the dims): G (M x npad: A, then Q1's vectors and R1), the
-// left vectors of a wide A (M x npad), X (Q2's), Y, V and the right vectors (npad x npad), the panels' T factors, and the
-// norms and orders.
-int64_t svd_scratch_bytes(int64_t m, int64_t n, int64_t esize) {
-    const int64_t M = std::max(m, n), N = std::min(m, n);
-    const int64_t npad = (N + JP - 1) / JP * JP;
-    const int64_t ldg  = (M + 1) / 2 * 2;
-    return esize * (2 * ldg * npad + 4 * npad * npad + 2 * QW * npad) + 8 * (2 * npad + 64) + 4 * (3 * npad + 64) + 256;
-}
-
 // Rank rule of svd.cpp:257-280 on descending sigma (only exactly-nonzero values count, like
 // svd_lapacke.cpp:453 S.nonZeros()).  Returns rank (>0) or -1 (the reference throws there).
 int64_t truncation_rank(const double *S, int64_t n, int64_t rank_max, int64_t rank_min, double lim, double *trunc_err) {
@@ -1131,6 +1121,23 @@ static int svd_factors(int64_t M, int64_t N) {
     if(M > QrPanel<T>::ROWS_MAX) return 0;
     if(N > QW + 1 || (N > QW && M > JW_ROWS) || (N >= 10 && M > 256)) return 2;
     return M > (N == 1 ? 256 : JW_ROWS) ? 1 : 0;
+}
+
+// Scratch of one SVD, in its tall orientation (M = max, N = min of the dims): G (M x npad: A, then Q1's vectors and R1) and V
+// (npad x npad); with factors Y (npad x npad: Jacobi's matrix, then the right vectors), the panels' T factors and, for a wide A, Z
+// (M x npad: A^H, then the left vectors); with two also X (npad x npad: Q2's vectors); the norms and orders.
+static int64_t svd_bytes(int64_t M, int64_t N, int qr, bool wide, int64_t esize) {
+    const int64_t npad = (N + JP - 1) / JP * JP, ldg = (M + 1) / 2 * 2;
+    return esize * (ldg * npad * (qr && wide ? 2 : 1) + npad * npad * (1 + qr) + (qr ? 2 * QW * npad : 0)) + 8 * (2 * npad + 64) + 4 * (3 * npad + 64) + 256;
+}
+int64_t svd_scratch_bytes(int64_t m, int64_t n, int64_t esize) {
+    const int64_t M = std::max(m, n), N = std::min(m, n);
+    return svd_bytes(M, N, esize == 16 ? svd_factors<double2>(M, N) : svd_factors<double>(M, N), m < n, esize);
+}
+// Enough for every matrix of up to m rows and n columns (a workspace that serves many shapes).
+int64_t svd_scratch_max(int64_t m, int64_t n, int64_t esize) {
+    const int64_t M = std::max(m, n), N = std::min(m, n), Mq = std::min<int64_t>(M, esize == 16 ? QrPanel<double2>::ROWS_MAX : QrPanel<double>::ROWS_MAX);
+    return std::max(svd_bytes(M, N, 0, false, esize), svd_bytes(Mq, std::min(N, Mq), 2, true, esize));
 }
 
 // In-place QR of G (M x N, leading dim ldg); the panels' T factors go to Tf (QW x QW each).
@@ -1186,14 +1193,15 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     const int     M = (int)std::max(m, n), N = (int)std::min(m, n);
     const int     npad = (N + JP - 1) / JP * JP;
     const int64_t ldg  = (M + 1) / 2 * 2;
+    const int     qr   = svd_factors<T>(M, N);
+    const bool    precond = qr > 0;
     T            *G    = reinterpret_cast<T *>(scratch);
     T            *Z    = G + ldg * npad;
-    T            *X    = Z + ldg * npad;
-    T            *Y    = X + (int64_t)npad * npad;
-    T            *V    = Y + (int64_t)npad * npad;
-    T            *R    = V + (int64_t)npad * npad;
-    T            *T1 = R + (int64_t)npad * npad, *T2 = T1 + QW * npad;
-    double       *sig  = reinterpret_cast<double *>(T2 + QW * npad);  // column norms
+    T            *V    = Z + (precond && wide ? ldg * npad : 0);
+    T            *Y    = V + (int64_t)npad * npad;
+    T            *X    = Y + (precond ? (int64_t)npad * npad : 0);
+    T            *T1 = X + (qr == 2 ? (int64_t)npad * npad : 0), *T2 = T1 + (precond ? QW * npad : 0);
+    double       *sig  = reinterpret_cast<double *>(T2 + (precond ? QW * npad : 0));  // column norms
     double       *dmax = sig + npad;  // [0] largest squared column norm of a sweep; [1] (int) pairs rotated in it, or sweeps run
     int          *drot = reinterpret_cast<int *>(dmax + 1);
     double       *sig0 = dmax + 64;   // norms of A's columns
@@ -1205,8 +1213,6 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
         HEFF_CUDA((launch_chained(col_order_kernel, (cols + 127) / 128, 128, 0, s, nrm, cols, ord)));
         return HEFF_OK;
     };
-    const int     qr   = svd_factors<T>(M, N);
-    const bool    precond = qr > 0;
     T            *W    = precond ? Y : G;  // the matrix Jacobi works on, rows x npad
     const int64_t ldw  = precond ? npad : ldg;
     const int     rows = precond ? N : M;
@@ -1322,7 +1328,10 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
     } else {
         T            *left = wide ? Z : U;
         const int64_t ldl  = wide ? ldg : M;
-        HEFF_CUDA((launch_chained(take_columns_kernel<T, false, false>, gr, 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, left, ldl, M, R, npad)));
+        // the right vectors take the place of the columns that the left ones come from
+        T *R = Y;
+        HEFF_CUDA((launch_chained(take_columns_kernel<T, false, false>, g1((int64_t)M * r), 256, 0, s, W, ldw, rows, V, npad, 0, perm, sig, kk, S, left, ldl, M, R, npad)));
+        HEFF_CUDA((launch_chained(take_columns_kernel<T, false, false>, g1((int64_t)N * r), 256, 0, s, W, ldw, rows, V, npad, N, perm, sig, kk, S, left, ldl, 0, R, npad)));
         HEFF_TRY(qr_apply_q<T>(G, ldg, M, N, T1, left, ldl, kk, s));
         HEFF_TRY(qr_apply_q<T>(X, npad, N, N, T2, R, npad, kk, s));
         if(!wide) {
@@ -1370,10 +1379,16 @@ __global__ void schmidt_unpack_kernel(const T *__restrict__ VT, T *__restrict__ 
     }
 }
 
-int64_t schmidt_scratch_bytes(int64_t dL, int64_t dR, int64_t cL, int64_t cR, int64_t rank_max, int64_t esize) {
-    const int64_t m = dL * cL, n = dR * cR;
+// for the split of one theta, and of every theta of up to these bonds
+static int64_t schmidt_bytes(int64_t m, int64_t n, int64_t rank_max, int64_t svd, int64_t esize) {
     const int64_t kmax = std::min(std::min(m, n), rank_max > 0 ? rank_max : INT64_MAX);
-    return esize * ((m * n + 31) / 32 * 32 + (kmax * n + 31) / 32 * 32) + svd_scratch_bytes(m, n, esize) + 512;
+    return esize * ((m * n + 31) / 32 * 32 + (kmax * n + 31) / 32 * 32) + svd + 512;
+}
+int64_t schmidt_scratch_bytes(int64_t dL, int64_t dR, int64_t cL, int64_t cR, int64_t rank_max, int64_t esize) {
+    return schmidt_bytes(dL * cL, dR * cR, rank_max, svd_scratch_bytes(dL * cL, dR * cR, esize), esize);
+}
+int64_t schmidt_scratch_max(int64_t dL, int64_t dR, int64_t cL, int64_t cR, int64_t rank_max, int64_t esize) {
+    return schmidt_bytes(dL * cL, dR * cR, rank_max, svd_scratch_max(dL * cL, dR * cR, esize), esize);
 }
 
 template<class T>
