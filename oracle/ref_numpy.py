@@ -359,7 +359,7 @@ def round_robin_pair(n, step, k):
 
 
 def jacobi_small_model(A, max_sweeps=60):
-    """Host model of the single-CTA one-sided Jacobi SVD (jacobi_small_kernel) in its index maps: the columns padded
+    """One-sided Jacobi SVD by direct rotations of column pairs, over the device kernels' tournament: the columns padded
     to a multiple of 32 (zeros), the tournament over the n columns rounded up to even, steps of disjoint pairs; per
     pair the squared norms app, aqq and apq = a_p^H a_q, skipped unless |apq| > max(1e-300, floor,
     tol sqrt(app aqq)) with tol = max(1e-14, 8 eps sqrt(m)) and floor = m eps^2 max ||G_j||^2 of the previous sweep
@@ -406,3 +406,89 @@ def jacobi_small_model(A, max_sweeps=60):
         floor = m * eps * eps * gmax
     sig = np.sort(np.linalg.norm(G, axis=0))[::-1]
     return sig[: min(m, n)], G, V, sweeps
+
+
+def jacobi_rotation(app, aqq, apq, tol, floor):
+    """(p, s e) of the rotation that annihilates apq = |apq| e in [[app, apq], [conj(apq), aqq]], in the device kernels' formula:
+    cosine c and sine s of the angle from those of twice the angle, p = s^2 / (1 + c) = 1 - c; zeros unless
+    |apq|^2 > max(floor^2, tol^2 |app aqq|), all of it scaled by 2^-exponent of the larger diagonal entry."""
+    sc = 2.0 ** -np.floor(np.log2(max(abs(app), abs(aqq), 1e-300)))
+    a, b, z, fl = app * sc, aqq * sc, apq * sc, floor * sc
+    h2 = abs(z) ** 2
+    if not (h2 > fl * fl and h2 > tol * tol * abs(a * b)):
+        return 0.0, 0.0
+    x = 0.5 * (b - a)
+    w = np.sqrt(x * x + h2)
+    c = np.sqrt(0.5 + 0.5 * abs(x) / w)
+    q = np.copysign(0.5 / (w * c), x)
+    s = np.sqrt(h2) * q
+    return s * s / (1.0 + c), z * q
+
+
+def gram_jacobi_sweep(G, nc, tol, floor):
+    """One cyclic two-sided Jacobi sweep of the Hermitian G over its first nc (even) columns, as JBlock::sweep runs it: nc - 1
+    steps of nc / 2 disjoint rotations, all of a step taken from the same G.  Returns (Q, rotated)."""
+    P = G.shape[0]
+    G = G.copy()
+    Q = np.eye(P, dtype=G.dtype)
+    rotated = False
+    for step in range(nc - 1):
+        J = np.eye(P, dtype=G.dtype)
+        for k in range(nc // 2):
+            a, b = round_robin_pair(nc, step, k)
+            p, se = jacobi_rotation(G[a, a].real, G[b, b].real, G[a, b], tol, floor)
+            if p != 0.0:
+                rotated = True
+                J[a, a] = J[b, b] = 1.0 - p
+                J[a, b], J[b, a] = se, -np.conj(se)
+        G = J.conj().T @ (G @ J)
+        Q = Q @ J
+    return Q, rotated
+
+
+def jacobi_gram_model(A, max_sweeps=60):
+    """Host model of the one-CTA device SVD (jacobi_whole_kernel and the factorisations before it) for at most 64 columns in its
+    tall orientation.  Two factorisations from 18 columns on (17 beyond 64 rows, 10 beyond 256): A P = Q1 R1 (columns by descending
+    norm), R1^H = Q2 R2, Y = R2^H; one beyond 64 rows (256 for a single column): A = Q1 R1, Y = R1; else Y = A.  Then sweeps over all
+    columns as one block: the Gram of Y, done when no off-diagonal of it exceeds max(tol sqrt(g_ii g_jj), floor), tol =
+    max(1e-14, 8 eps sqrt(rows of A)), floor = rows eps^2 max g_ii of the previous sweep (0 in the first); else one two-sided sweep
+    on the Gram with half of both thresholds, Y <- Y Q, V <- V Q.
+    Returns (U, sigma descending, V, sweeps) with A = U diag(sigma) V^H; columns of U for sigma = 0 are zero."""
+    wide = A.shape[0] < A.shape[1]
+    B = A.conj().T if wide else A
+    m, n = B.shape
+    P, nc = (n + 31) // 32 * 32, (n + 1) // 2 * 2
+    factors = 2 if n > 17 or (n > 16 and m > 64) or (n >= 10 and m > 256) else int(m > (256 if n == 1 else 64))
+    order = np.argsort(-np.linalg.norm(B, axis=0), kind="stable") if factors == 2 else np.arange(n)
+    Q1, Q2, Y0 = None, np.eye(n), B
+    if factors:
+        Q1, Y0 = np.linalg.qr(B[:, order])
+    if factors == 2:
+        Q2, R2 = np.linalg.qr(Y0.conj().T)
+        Y0 = R2.conj().T
+    rows = Y0.shape[0]
+    Y = np.zeros((rows, P), dtype=np.complex128 if np.iscomplexobj(A) else np.float64)
+    Y[:, :n] = Y0
+    V = np.eye(P, dtype=Y.dtype)
+    eps = 2.220446049250313e-16
+    tol, floor, sweeps = max(1e-14, 8.0 * eps * np.sqrt(m)), 0.0, max_sweeps
+    for sweep in range(max_sweeps):
+        G = Y.conj().T @ Y
+        d = np.abs(np.diag(G).real)
+        off = np.abs(np.triu(G, 1))[:nc, :nc]
+        if not np.any((off > floor) & (off > tol * np.sqrt(np.outer(d, d))[:nc, :nc])):
+            sweeps = sweep + 1
+            break
+        Q, _ = gram_jacobi_sweep(G, nc, 0.5 * tol, 0.5 * floor)
+        Y, V = Y @ Q, V @ Q
+        floor = rows * eps * eps * float(d.max())
+    sig = np.linalg.norm(Y, axis=0)
+    perm = np.argsort(-sig, kind="stable")[:n]
+    sig = sig[perm]
+    U = np.divide(Y[:, perm], sig, out=np.zeros_like(Y[:, perm]), where=sig > 0)
+    V = V[:n, perm]
+    U = Q1 @ U if factors else U
+    W = np.empty_like(V)
+    W[order] = Q2 @ V
+    V = W
+    return (V, sig, U, sweeps) if wide else (U, sig, V, sweeps)
