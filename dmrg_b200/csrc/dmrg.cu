@@ -491,8 +491,8 @@ static int gemm_nn(const double *A, int64_t lda, const double *B, int64_t ldb, d
     return gemm_f64<false>(false, false, g, s);
 }
 
-// A (m x n, lda) = U S VT with U m x k (ld m), VT k x n (ld k); the one-sided Jacobi always runs on the taller
-// orientation (a wide matrix is transposed first and the factors swapped back).
+// A (m x n, lda) = U S VT with U m x k (ld m), VT k x n (ld k).  A wide A is transposed first, into buffers that the sweep has
+// anyway, and the factors are swapped back.
 static int svd_oriented(DmrgWorkspace &ws, const double *A, int64_t lda, int64_t m, int64_t n, int64_t rank_max, double trunc, double *U, double *S,
                         double *VT, int64_t *k, double *err, cudaStream_t s) {
     if(m >= n) return svd_truncated(A, lda, m, n, rank_max, trunc, U, S, VT, k, err, ws.escr, nullptr, s);

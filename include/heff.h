@@ -140,7 +140,11 @@ int heff_expansion_term_z(int side, heff_z *P, const heff_z *env, const int64_t 
  * at most rank_max (<= 0: no limit).  U [rows x k], S [k] (not normalised, like
  * svd_lapacke.cpp:457), VT [k x cols] are device buffers sized for
  * k = min(rows, cols, rank_max); *rank and *trunc_err are host outputs.
- * Synchronises the stream. */
+ * Jacobi runs on triangular factors of A where that pays: from 18 columns (of the
+ * tall orientation) or 65 rows on, up to 5376 rows (complex 3584).  Longer matrices
+ * are rotated as they are, in two to five times as many sweeps.  Scratch, kept per
+ * stream: A and one square of the shorter side, with factors one or two squares
+ * more and, for rows < cols, A once more.  Synchronises the stream. */
 int heff_svd_d(const double *A, int64_t rows, int64_t cols, int64_t rank_max, double trunc_lim, double *U, double *S, double *VT, int64_t *rank,
                double *trunc_err, void *stream);
 /* Two-site Schmidt split, replacing svd::solver::schmidt_multisite
@@ -206,14 +210,18 @@ int64_t heff_op_num_mv(const heff_op *op);
 /* Stage timing (the reference's tid:: timers around MultAx, matvec_mpo.h:70-102):
  * when enabled, every FP64 matvec records CUDA events around its four kernels
  * (layout, GEMM 1, MPO mix, GEMM 2).  heff_op_stage_times synchronises the op's
- * stream and returns the summed milliseconds per stage and the matvec count. */
+ * stream and returns the summed milliseconds per stage and the matvec count.
+ * Small bonds, whose product is otherwise one launch, run as four kernels too while
+ * it is enabled: their stages then add up to more than that launch takes, and the
+ * result differs from its at the rounding level. */
 int heff_op_set_profiling(heff_op *op, int enable);
 /* CUDA graphs for the FP64 matvec (off by default, or on for every operator when the
  * environment variable HEFF_GRAPHS=1; no counterpart in the reference):
  * on an operator created with a non-default stream, the first product of a shape
  * runs as plain kernel launches and is recorded as a graph; later products of that
  * shape replay it with the input and output retargeted (one launch instead of
- * four to six).  Results are bitwise identical either way.  0 turns it off. */
+ * four to six).  Products of small bonds are one launch already and are not
+ * recorded.  Results are bitwise identical either way.  0 turns it off. */
 int heff_op_set_graphs(heff_op *op, int enable);
 int heff_op_stage_times(heff_op *op, double ms[4], int64_t *count, int reset);
 /* Device-side status of the operator's tensor-core pipeline: *code = 0 when every
