@@ -1131,9 +1131,9 @@ static int64_t svd_bytes(int64_t M, int64_t N, int qr, bool wide, int64_t esize)
     const int64_t npad = (N + JP - 1) / JP * JP, ldg = (M + 1) / 2 * 2;
     return esize * (ldg * npad * (qr && wide ? 2 : 1) + npad * npad * (1 + qr) + (qr ? 2 * QW * npad : 0)) + 8 * (2 * npad + 64) + 4 * (3 * npad + 64) + 256;
 }
-int64_t svd_scratch_bytes(int64_t m, int64_t n, int64_t esize) {
+int64_t svd_scratch_bytes(int64_t m, int64_t n, int64_t esize, bool flat) {
     const int64_t M = std::max(m, n), N = std::min(m, n);
-    return svd_bytes(M, N, esize == 16 ? svd_factors<double2>(M, N) : svd_factors<double>(M, N), m < n, esize);
+    return svd_bytes(M, N, flat ? 0 : (esize == 16 ? svd_factors<double2>(M, N) : svd_factors<double>(M, N)), m < n, esize);
 }
 // Enough for every matrix of up to m rows and n columns (a workspace that serves many shapes).
 int64_t svd_scratch_max(int64_t m, int64_t n, int64_t esize) {
@@ -1184,17 +1184,18 @@ static int jacobi_attributes() {
 }
 
 // Full SVD driver.  A: m x n (lda), not modified.  Outputs (device): U (m x kmax), S (kmax), VT (kmax x n)
-// with kmax = min(m, n, rank_max>0 ? rank_max : inf); *rank and *trunc_err on the host.
+// with kmax = min(m, n, rank_max>0 ? rank_max : inf); *rank and *trunc_err on the host.  flat: the caller knows that the
+// singular values lie close together, so factors would save no sweeps.
 template<class T>
 static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_t rank_max, double trunc_lim, T *U, double *S, T *VT, int64_t *rank,
-                           double *trunc_err, void *scratch, int *sweeps_out, cudaStream_t s) {
+                           double *trunc_err, void *scratch, int *sweeps_out, cudaStream_t s, bool flat = false) {
     if(m <= 0 || n <= 0 || m > (1 << 24) || n > 16384) return HEFF_BAD_SHAPE;
     HEFF_TRY(jacobi_attributes<T>());
     const bool    wide = m < n;  // worked on as A^H
     const int     M = (int)std::max(m, n), N = (int)std::min(m, n);
     const int     npad = (N + JP - 1) / JP * JP;
     const int64_t ldg  = (M + 1) / 2 * 2;
-    const int     qr   = svd_factors<T>(M, N);
+    const int     qr   = flat ? 0 : svd_factors<T>(M, N);
     const bool    precond = qr > 0;
     T            *G    = reinterpret_cast<T *>(scratch);
     T            *Z    = G + ldg * npad;
@@ -1348,12 +1349,12 @@ static int svd_truncated_t(const T *A, int64_t lda, int64_t m, int64_t n, int64_
 }
 
 int svd_truncated(const double *A, int64_t lda, int64_t m, int64_t n, int64_t rank_max, double trunc_lim, double *U, double *S, double *VT,
-                  int64_t *rank, double *trunc_err, void *scratch, int *sweeps_out, cudaStream_t s) {
-    return svd_truncated_t<double>(A, lda, m, n, rank_max, trunc_lim, U, S, VT, rank, trunc_err, scratch, sweeps_out, s);
+                  int64_t *rank, double *trunc_err, void *scratch, int *sweeps_out, cudaStream_t s, bool flat) {
+    return svd_truncated_t<double>(A, lda, m, n, rank_max, trunc_lim, U, S, VT, rank, trunc_err, scratch, sweeps_out, s, flat);
 }
 int svd_truncated(const double2 *A, int64_t lda, int64_t m, int64_t n, int64_t rank_max, double trunc_lim, double2 *U, double *S, double2 *VT,
-                  int64_t *rank, double *trunc_err, void *scratch, int *sweeps_out, cudaStream_t s) {
-    return svd_truncated_t<double2>(A, lda, m, n, rank_max, trunc_lim, U, S, VT, rank, trunc_err, scratch, sweeps_out, s);
+                  int64_t *rank, double *trunc_err, void *scratch, int *sweeps_out, cudaStream_t s, bool flat) {
+    return svd_truncated_t<double2>(A, lda, m, n, rank_max, trunc_lim, U, S, VT, rank, trunc_err, scratch, sweeps_out, s, flat);
 }
 
 // theta [dL*dR, chiL, chiR] -> A[(s1 + dL a), (s2 + dR b)] = theta[s1 + dL s2, a, b]   (svd.h:217 reshape+shuffle)
