@@ -118,17 +118,6 @@ __device__ __forceinline__ void dmma_f64(double (&c)[4], double a0, double a1, d
                  : "d"(a0), "d"(a1), "d"(b0));
 }
 
-__device__ __forceinline__ float rcp_fast(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-// 1 / d for d in [1, 2]: a single-precision reciprocal and two Newton steps (relative error a few eps).
-__device__ __forceinline__ double rcp_near_one(double d) {
-    double r = (double)rcp_fast((float)d);
-    r        = fma(r, fma(-d, r, 1.0), r);
-    return fma(r, fma(-d, r, 1.0), r);
-}
 // 2^-exponent of the larger diagonal entry: scaled by it, the squares below stay in range whatever the matrix's scale.
 __device__ __forceinline__ double pair_scale(double app, double aqq) {
     const int ex = (__double2hiint(fmax(fabs(app), fabs(aqq))) >> 20) & 0x7ff;
@@ -158,7 +147,11 @@ __device__ __forceinline__ bool jacobi_rotation(double app, double aqq, T apq, d
     if(!significant(a, b, z, tol, fl)) return false;
     const double x = 0.5 * (b - a), h2 = JS<T>::abs2(z);
     const double rw = rsqrt(fma(x, x, h2)), v = fma(0.5 * fabs(x), rw, 0.5), rc = rsqrt(v);  // v = c^2
-    const double q = copysign(0.5 * rw * rc, x), rd = rcp_near_one(fma(v, rc, 1.0));
+    const double q = copysign(0.5 * rw * rc, x), d = fma(v, rc, 1.0);
+    // 1 / (1 + c): the cubic in v with the smallest relative error on [1/2, 1] (8e-5), which does not wait for c, and two Newton steps
+    double rd = fma(fma(fma(-0.094144, v, 0.323722), v, -0.49239), v, 0.762772);
+    rd        = fma(rd, fma(-d, rd, 1.0), rd);
+    rd        = fma(rd, fma(-d, rd, 1.0), rd);
     double       sn;
     if constexpr(std::is_same<T, double>::value) {
         se = z * q;
