@@ -8,7 +8,7 @@
 // take one factorisation or none, svd_factors):
 //   A P = Q1 R1,   R1^H = Q2 R2,   Y = R2^H = U_j S V_j^H (Jacobi),   A = (Q1 U_j) S (P Q2 V_j)^H.
 // The two factorisations push Y close to diagonal, so Jacobi needs 5-9 sweeps on n x n instead of 10-35 on m x n (dense
-// graded spectra most: 28 -> 6 in a host model at n = 256).  Measured, graded spectrum: 512 x 512 72 -> 8.0 ms, 2048 x 2048
+// graded spectra most: 28 -> 6 in a host model at n = 256).  Measured, graded spectrum: 512 x 512 72 -> 7.9 ms, 2048 x 2048
 // 1270 -> 88 ms, complex 70 x 172 23 -> 1.4 ms, 64 x 64 3.4 -> 0.66 ms, 32 x 32 0.82 -> 0.28 ms.
 //
 // Jacobi: the columns of the work matrix (Y, npad columns, n padded to a multiple of 32 with zero columns) are ordered by
